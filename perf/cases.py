@@ -3,10 +3,9 @@
 A case is a dict of plain values; ``prepare`` makes what the program has in
 hand (the tilt series, the geometry, buffers) and ``run`` is one pass through
 ``autom2_b200.tiltrec``.  As a program that reconstructs series after series
-does, one Engine (and one Scheduler) is kept per process: a pass hands it the
-series' geometry -- ``update_geometry`` for a series of the shape already set,
-``set_problem`` for another shape -- and then calls the method, so that
-geometry-dependent weights belong to the pass.
+does, one Engine (and one Scheduler) is kept per process: a pass sets the
+series' problem on it and then calls the method, so that geometry-dependent
+weights belong to the pass.
 
 Kinds:
 
@@ -162,6 +161,7 @@ def prepare(case, seed):
             s["series"].append(dict(coeff=_coeffs(j, rng), proj=_stack(j, gen), layout=j["layout"],
                                     vol=torch.zeros(_vol_shape(j), device="cuda")))
         _scheduler()
+        torch.cuda.synchronize()  # the scheduler's streams are its own
         return s
     s["coeff"] = _coeffs(case, rng)
     if kind == "project":
@@ -173,7 +173,7 @@ def prepare(case, seed):
         s["vol"] = torch.zeros(_vol_shape(case), device="cuda")
         if kind in ("wbp", "fbp"):
             s["rows"] = torch.empty_like(s["proj"])
-    _problem(case, s["coeff"])
+    _engine()
     return s
 
 
@@ -193,13 +193,9 @@ def _scheduler():
 
 
 def _problem(case, coeff):
-    """The process's Engine, set to the series' geometry."""
+    """The process's Engine, set to the series."""
     e = _engine()
-    shape = (case["nx"], case["ny"], case["nt"], case["th"], case["layout"])
-    if e.shape == shape:
-        e.update_geometry(coeff)
-    else:
-        e.set_problem(case["nx"], case["ny"], case["nt"], case["th"], coeff, case["layout"])
+    e.set_problem(case["nx"], case["ny"], case["nt"], case["th"], coeff, case["layout"])
     return e
 
 
