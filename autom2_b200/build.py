@@ -27,7 +27,7 @@ BINDIR = os.path.join(PKG, "bin")
 LIB = os.path.join(LIBDIR, "libtiltrec_b200.so")
 
 GENCODE = ["-gencode", "arch=compute_100a,code=sm_100a"]
-CU_SOURCES = ["tr_kernels.cu", "tr_filter.cu", "tr_api.cu", "tr_static.cu", "tr_sched.cu",
+CU_SOURCES = ["tr_kernels.cu", "tr_rows.cu", "tr_filter.cu", "tr_api.cu", "tr_static.cu", "tr_sched.cu",
               "tr_admm.cu", "tr_output.cu"]
 CLI_SOURCES = ["mrc_io.cpp", "tiltrec_cli.cpp"]
 
@@ -73,6 +73,7 @@ def _build_to(out: str, cmd_for) -> None:
 def build_lib(force: bool = False, verbose_ptxas: bool = False) -> str:
     srcs = [os.path.join(CSRC, s) for s in CU_SOURCES]
     deps = srcs + [os.path.join(CSRC, "tr_internal.cuh"), os.path.join(CSRC, "tr_geom.h"),
+                   os.path.join(CSRC, "tr_device.cuh"),
                    os.path.join(CSRC, "tr_filter_host.h"),
                    os.path.join(INCLUDE, "tiltrec_b200.h")]
     if not force and _newer(LIB, deps):

@@ -51,6 +51,7 @@ struct tr_ctx {
   struct Slot {
     size_t cap = 0;
     unsigned gen = 0;
+    bool optional = false;  // may be dropped for a buffer that a call cannot do without
   };
   std::map<void **, Slot> slots;
   unsigned gen = 0;
@@ -89,6 +90,12 @@ struct tr_ctx {
   bool deterministic = false;
   unsigned long long *ival_d = nullptr;
   unsigned *gmax_d = nullptr;
+  // row-invariant geometries: the back-projection's voxel-row stack and the
+  // forward projection's row sums, and the last use of either
+  bool rows = false;
+  int rbp_cols = 0, rfp_cols = 0;
+  float *rows_d = nullptr, *rowsum_d = nullptr;
+  cudaEvent_t ev_rows = nullptr;
   cudaStream_t cp_in = nullptr, cp_out = nullptr;
   cudaEvent_t ev_in[3] = {}, ev_comp[3] = {}, ev_free[3] = {}, ev_start = nullptr;
 };
@@ -137,10 +144,11 @@ void scratch_free(tr_ctx *c, void **p) {
   sl.cap = 0;
 }
 
-// Frees the scratch buffers no call of the current problem has claimed.
+// Frees the scratch buffers no call of the current problem has claimed, and
+// the optional ones (cudaFree waits for the work that uses them).
 void release_idle(tr_ctx *c) {
   for (auto &kv : c->slots)
-    if (*kv.first && kv.second.gen != c->gen) scratch_free(c, kv.first);
+    if (*kv.first && (kv.second.gen != c->gen || kv.second.optional)) scratch_free(c, kv.first);
 }
 
 // Claims scratch buffer *p with at least `bytes` for the current problem:
@@ -174,6 +182,26 @@ tr_status scratch_alloc(tr_ctx *c, void **p, size_t bytes, const char *what) {
   sl.gen = c->gen;
   c->scratch += bytes;
   return TR_OK;
+}
+
+// As scratch_alloc for a buffer that the call can do without: false, with
+// nothing released and no error left, when the budget or the device has no room.
+bool scratch_try(tr_ctx *c, void **p, size_t bytes) {
+  tr_ctx::Slot &sl = c->slots[p];
+  sl.optional = true;
+  if (!*p || sl.cap < bytes) {
+    if (c->budget && c->scratch - (*p ? sl.cap : 0) + bytes > c->budget) return false;
+    if (*p) scratch_free(c, p);
+    if (cudaMalloc(p, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      *p = nullptr;
+      return false;
+    }
+    sl.cap = bytes;
+    c->scratch += bytes;
+  }
+  sl.gen = c->gen;
+  return true;
 }
 
 // Ends the current problem.  Its scratch buffers stay allocated for the next
@@ -231,11 +259,65 @@ BpArgs bp_args(const tr_ctx *c, float *vol, int z0, int nz, const float *img,
   return a;
 }
 
+// Row-invariant path (tr_rows.cu) for a launch over nz sections and nt tilts on
+// `s`.  Its tiles are 16 x 128 x 8 voxels where the general kernels' are
+// (general_x) x 4 x 32, so it takes the launches whose padding to its tiles
+// (most of all of the rows to 128) does not outweigh its gain -- `pad` bounds
+// the padded voxels relative to the general kernels' -- and which have tiles
+// enough for the SMs.  Measured (us, general / row-invariant):
+//   back-projection, pad 1.35, 128 tiles: 1024 x 1024 x 256, 61 tilts 6686 /
+//     3833; x 64, 1 tilt 320 / 147; 256 x 256 x 64, 41 tilts 91 / 68; rows 192
+//     of 256 (pad 1.33) 182 / 165, 160 of 256 (1.6) 110 / 116; 256 x 64 x 64
+//     (64 tiles, pad 2) 37 / 48;
+//   forward projection, pad 1.15, 256 tiles: 1024 x 1024 x 256, 61 tilts 8123 /
+//     6071; x 64: 41 tilts 1408 / 1280, 24 tilts 820 / 826, 8 tilts 305 / 459
+//     (the tilts pass through a CTA's warps in a pipeline that must fill);
+//     256 x 256 x 64 125 / 100, x 32 (128 tiles) 99 / 112; rows 320 of 384
+//     (pad 1.2) 355 / 391.
+// Not under stream capture, whose graphs must not hold a buffer that the
+// context may drop.
+struct RowsRule {
+  int general_x, min_tilts, min_tiles;
+  double pad;
+};
+constexpr RowsRule kRowsBp{kTX, 1, 128, 1.35}, kRowsFp{kFX, 24, 256, 1.15};
+bool rows_path(const tr_ctx *c, const RowsRule &r, int nz, int nt, cudaStream_t s) {
+  if (!c->rows || nt < r.min_tilts) return false;
+  const auto tiles = [](int n, int t) { return (double)((n + t - 1) / t); };
+  const double n = tiles(c->nx, kRowBpX) * tiles(c->ny, kRowTile) * tiles(nz, kRowBpZ);
+  const double general = tiles(c->nx, r.general_x) * r.general_x * tiles(c->ny, kTY) * kTY *
+                         tiles(nz, kTZ) * kTZ;
+  if (n < r.min_tiles || n * kRowBpX * kRowTile * kRowBpZ > r.pad * general) return false;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return cs == cudaStreamCaptureStatusNone;
+}
+static_assert(kRowBpX == kRowFpX && kRowBpZ == kRowFpZ && kTZ == kFTZ, "one tile for the rule");
+// Orders `s` after the row buffers' last use, on whichever stream that was, and
+// marks their use so far on `s` as the last.
+cudaError_t rows_acquire(tr_ctx *c, cudaStream_t s) {
+  if (!c->ev_rows) return cudaEventCreateWithFlags(&c->ev_rows, cudaEventDisableTiming);
+  return cudaStreamWaitEvent(s, c->ev_rows, 0);
+}
+cudaError_t rows_release(tr_ctx *c, cudaStream_t s) { return cudaEventRecord(c->ev_rows, s); }
+
 // Back-projection launch: clears the launch-wide abort word first.
 cudaError_t run_bp(tr_ctx *c, int mode, const BpArgs &a, cudaStream_t s) {
-  if (c->err_d) {
-    cudaError_t e = cudaMemsetAsync(c->err_d, 0, sizeof(int), s);
-    if (e != cudaSuccess) return e;
+  cudaError_t e;
+  if (c->err_d && (e = cudaMemsetAsync(c->err_d, 0, sizeof(int), s)) != cudaSuccess) return e;
+  if ((mode == BP_NORM || (mode == BP_SIRT && a.wslot) || mode == BP_SUM) && a.img.dtype == IMG_F32 && c->err_d &&
+      rows_path(c, kRowsBp, a.v.nz, a.nt, s) && bp_rows_fits(c->rbp_cols, a.nt) &&
+      scratch_try(c, (void **)&c->rows_d,
+                  row_stack_floats(c->nx, c->ny, a.t0 + a.nt, c->rbp_cols) * sizeof(float))) {
+    if ((e = rows_acquire(c, s)) != cudaSuccess ||
+        (e = launch_blend_rows(a.img, a.geo, a.t0, a.nt, a.oy, c->ny, c->rbp_cols, mode == BP_NORM,
+                               c->rows_d, s)) != cudaSuccess ||
+        (e = launch_bp_rows(mode, a, c->rows_d, c->rbp_cols, s)) != cudaSuccess)
+      return e;
+    return rows_release(c, s);
   }
   return launch_bp(mode, c->sep, a, s);
 }
@@ -271,6 +353,7 @@ FpArgs fp_args(const tr_ctx *c, const float *vol, int z0, int nz, float *val,
   a.fh = c->ffh;
   a.chunk = c->chunk_fp;
   a.nbound = c->fp_nbound;
+  a.err = c->err_d;
   return a;
 }
 
@@ -278,6 +361,19 @@ FpArgs fp_args(const tr_ctx *c, const float *vol, int z0, int nz, float *val,
 // tr_set_deterministic the int64 one (sums cleared first, converted after).
 tr_status run_fp(tr_ctx *c, const FpArgs &a, cudaStream_t s) {
   if (!c->deterministic) {
+    const size_t rb =
+        row_stack_floats(c->nx, c->ny, a.t0 + a.nt, c->rfp_cols) * sizeof(float);
+    if (rows_path(c, kRowsFp, a.v.nz, a.nt, s) && fp_rows_fits(c->rfp_cols, a.nt) &&
+        scratch_try(c, (void **)&c->rowsum_d, rb)) {
+      TR_CUDA(c, rows_acquire(c, s));
+      TR_CUDA(c, cudaMemsetAsync(c->err_d, 0, sizeof(int), s));
+      TR_CUDA(c, cudaMemsetAsync(c->rowsum_d, 0, rb, s));
+      TR_CUDA(c, launch_fp_rows(a, c->rowsum_d, c->rfp_cols, c->nsm, s));
+      TR_CUDA(c, launch_unblend_rows(c->rowsum_d, a.geo, a.t0, a.nt, a.oy, c->ny, c->rfp_cols,
+                                     a.val, a.tstride, c->nx, c->ny, s));
+      TR_CUDA(c, rows_release(c, s));
+      return TR_OK;
+    }
     TR_CUDA(c, launch_fp(c->sep, a, s));
     return TR_OK;
   }
@@ -353,6 +449,9 @@ tr_status load_geometry(tr_ctx *c, const double *coeff8, cudaStream_t s) {
   c->ffh = gi.ffh;
   c->fp_nbound = gi.nbound;
   c->sep = gi.sep;
+  c->rows = gi.rows;
+  c->rbp_cols = gi.rbp_cols;
+  c->rfp_cols = gi.rfp_cols;
   c->chunk_bp = chunk_for(kSmemBp, gi.bp_tilt_bytes);
   c->chunk_fp = chunk_for(kSmemFp, gi.fp_tilt_bytes);
   c->wt_ready = c->wtvol_ready = false;
@@ -742,6 +841,7 @@ tr_status tr_destroy(tr_ctx *c) {
     for (cudaEvent_t e : {c->ev_in[i], c->ev_comp[i], c->ev_free[i]})
       if (e) cudaEventDestroy(e);
   if (c->ev_start) cudaEventDestroy(c->ev_start);
+  if (c->ev_rows) cudaEventDestroy(c->ev_rows);
   if (c->err_d) cudaFree(c->err_d);
   delete c;
   return TR_OK;

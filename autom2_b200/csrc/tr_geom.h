@@ -16,6 +16,8 @@ struct GeomInfo {
   int ffw, ffh;    // forward-projection tile window
   float nbound;    // most voxel contributions one forward window entry collects
   bool sep;        // every tilt has b1 = b3 = 0, b2 = 1 (separable rows)
+  bool rows;       // row-invariant: every tilt has a2 = 0, 0 <= a1 <= 1, |a3| <= 1, and sep
+  int rbp_cols, rfp_cols;  // window columns of a row-invariant tile (tr_rows.cu)
   size_t fp_tilt_bytes;  // shared memory of one staged tilt's splat window
   size_t bp_tilt_bytes;  // shared memory of one staged tilt's interpolation table
 };
@@ -61,11 +63,17 @@ inline float fp_entry_bound_sep(double min_a1) {
   return (float)(n * kFTZ);
 }
 
+// Voxels along x and z of a row-invariant tile (tr_rows.cu): back-projection
+// and forward projection.
+constexpr int kRowBpX = 16, kRowBpZ = 8;
+constexpr int kRowFpX = 16, kRowFpZ = 8;
+
 // Fills g[0..nt) and *out from [nt][8] coefficients; *bad_tilt names the
 // offending tilt for the per-tilt failures.
 inline int derive_geometry(const double *coeff8, int nt, int nx, int ny, int th,
                            size_t smem_max, TiltGeo *g, GeomInfo *out, int *bad_tilt) {
-  bool sep = true;
+  bool sep = true, rows = true;
+  double rbp = 0, rfp = 0;
   double span_u = 0, span_v = 0, fspan_u = 0, fspan_v = 0, min_a1 = 1e30, sect = 0;
   const double two32 = 4294967296.0;
   const double ext = std::max(std::max(nx, ny), th) + 64.0;
@@ -91,6 +99,9 @@ inline int derive_geometry(const double *coeff8, int nt, int nx, int ny, int th,
         std::fabs(k[4]) + (std::fabs(k[5]) + std::fabs(k[6]) + std::fabs(k[7])) * 2 * ext;
     if (reach_u > 1.0e9 || reach_v > 1.0e9) return GEOM_RANGE;
     if (!(k[5] == 0.0 && k[7] == 0.0 && k[6] == 1.0)) sep = false;
+    if (!(k[2] == 0.0 && k[1] >= 0.0 && k[1] <= 1.0 && std::fabs(k[3]) <= 1.0)) rows = false;
+    rbp = std::max(rbp, std::fabs(k[1]) * (kRowBpX - 1) + std::fabs(k[3]) * (kRowBpZ - 1));
+    rfp = std::max(rfp, std::fabs(k[1]) * (kRowFpX - 1) + std::fabs(k[3]) * (kRowFpZ - 1));
     min_a1 = std::min(min_a1, std::fabs(k[1]));
     sect = std::max(sect, fp_section_bound(k[1], k[2], k[5], k[6]));
     span_u = std::max(span_u, std::fabs(k[1]) * (kTX - 1) + std::fabs(k[2]) * (kTY - 1) +
@@ -118,6 +129,12 @@ inline int derive_geometry(const double *coeff8, int nt, int nx, int ny, int th,
   out->ffh = sep ? kTY : (int)std::ceil(fspan_v) + 5;
   out->nbound = sep ? fp_entry_bound_sep(min_a1) : (float)(sect * kFTZ);
   out->sep = sep;
+  // A row-invariant tile's window starts at column floor(umin) - 1; its voxels
+  // reach lower columns up to floor(umax) and one more for the fixed-point
+  // coordinates, and the column above.
+  out->rows = sep && rows;
+  out->rbp_cols = (int)std::ceil(rbp) + 4;
+  out->rfp_cols = (int)std::ceil(rfp) + 4;
   out->fp_tilt_bytes = (size_t)out->ffw * out->ffh * sizeof(int);
   out->bp_tilt_bytes = (size_t)out->fw * out->fh * sizeof(float2);
   if (out->bp_tilt_bytes > smem_max || out->fp_tilt_bytes > smem_max) return GEOM_SMEM;

@@ -30,6 +30,11 @@ constexpr int kFTZ = kZG * kFNV;              // 32
 // coordinates in Q9.23 fixed point, whose integer part is below 512.
 constexpr int kMaxWindow = 511;
 
+// Row-invariant geometries (tr_rows.cu): rows of a tile, and the shared memory
+// a CTA may take, alone on its SM or as one of two.
+constexpr int kRowTile = 128;
+constexpr size_t kRowSmem = 220 * 1024, kRowSmem2 = 113 * 1024;
+
 // Per-tilt projection geometry.  a/b are the reference's linear coefficients
 // (detector x = a0 + a1 X + a2 Y + a3 Z + ox, y likewise with b, X/Y/Z the
 // voxel offsets from the origin).  A/B are the same slopes in Q32.32 fixed
@@ -114,6 +119,7 @@ struct FpArgs {
   unsigned long long *ival;
   const unsigned *gmax;
   double gbound;
+  int *err;           // row-invariant path: as BpArgs::err
 };
 
 // Footprint bookkeeping of one tilt for one tile, computed in FP64.
@@ -241,6 +247,30 @@ cudaError_t launch_fp(bool sep, const FpArgs &a, cudaStream_t s);
 // zero), then the sums converted and added into a.val.
 cudaError_t launch_fp_deterministic(bool sep, FpArgs a, unsigned long long *ival,
                                     unsigned *gmax, int nsm, cudaStream_t s);
+// Row-invariant geometries (tr_rows.cu).  A row stack holds [tilt][block of
+// kRowTile rows][column][row] floats, the columns with `margin` more on each
+// side of the detector's.
+inline size_t row_stack_floats(int nx, int ny, int nt, int margin) {
+  return (size_t)nt * ((ny + kRowTile - 1) / kRowTile) * kRowTile * (nx + 2 * (size_t)margin);
+}
+bool bp_rows_fits(int cols, int nt);
+bool fp_rows_fits(int cols, int nt);
+// Image stack -> voxel-row stack of tilts [t0, t0 + nt): norm, columns -1..nx of
+// the edge-clamped image normalised by the rows' in-image weight; else columns
+// 0..nx-1 of the in-image rows.
+cudaError_t launch_blend_rows(const ImgView &im, const TiltGeo *geo, int t0, int nt, float oy,
+                              int vny, int margin, bool norm, float *rows, cudaStream_t s);
+// Back-projection (BP_NORM, BP_SIRT or BP_SUM) from the row stack that
+// launch_blend_rows(margin = cols, norm = mode == BP_NORM) made; cols: the
+// tile's window.
+cudaError_t launch_bp_rows(int mode, const BpArgs &a, const float *rows, int cols, cudaStream_t s);
+// Forward projection added into a row stack of margin `cols`; a.val is not
+// used.
+cudaError_t launch_fp_rows(const FpArgs &a, float *rows, int cols, int nsm, cudaStream_t s);
+// Adds such a row stack into an image stack.
+cudaError_t launch_unblend_rows(const float *rows, const TiltGeo *geo, int t0, int nt, float oy,
+                                int vny, int margin, float *val, long long tstride, int nx, int ny,
+                                cudaStream_t s);
 cudaError_t launch_resid(const float *p, float *val, const float *wt, size_t n, int nsm,
                          cudaStream_t s);
 cudaError_t launch_quantize(const float *p, size_t plane, int nt, int dtype, void *out,

@@ -32,7 +32,6 @@
 // the two rows are blended while staging and the inner loop is one table
 // read and one FMA per voxel and tilt.
 #include <cuda.h>
-#include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <stdint.h>
@@ -41,6 +40,7 @@
 
 #include <algorithm>
 
+#include "tr_device.cuh"
 #include "tr_internal.cuh"
 
 namespace trb {
@@ -62,38 +62,6 @@ __device__ __forceinline__ float to_f(__nv_bfloat16 v) { return __bfloat162float
 // the rounded ones (the forward splat's fixed-point windows).
 constexpr int kFshiftBias = 0x4B400000;
 __device__ __forceinline__ int fshift(float x) { return __float_as_int(x + 12582912.0f); }
-
-// Paired FP32 arithmetic (sm_100 f32x2): two lanes of float math per
-// instruction on 64-bit register pairs {lo, hi}.
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(f32x2 r, float &lo, float &hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(r));
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
 
 __device__ __forceinline__ int clampi(int v, int lo, int hi) {
   return v < lo ? lo : (v > hi ? hi : v);
@@ -476,48 +444,6 @@ __global__ void __launch_bounds__(kThreads)
 // tensor needs 16-byte row strides, so this path serves images whose rows are
 // a multiple of 16 bytes (width % 4 for float, % 8 for 16-bit elements); the
 // others stage through bp_kernel.
-
-__device__ __forceinline__ unsigned smem_u32(const void *p) {
-  return (unsigned)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(unsigned long long *m, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(m)), "r"(count)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long *m, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(m)),
-               "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long *m, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(smem_u32(m)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Waits for a phase until it completes (true), `budget` clock cycles pass or
-// the launch-wide abort word becomes non-zero (false).
-__device__ __forceinline__ bool mbar_wait_bounded(unsigned long long *m, unsigned parity,
-                                                  long long budget, const int *abort_word) {
-  const long long t0 = clock64();
-  for (;;) {
-    if (mbar_try_wait(m, parity)) return true;
-    if (clock64() - t0 > budget) return false;
-    if (abort_word && *(volatile const int *)abort_word) return false;
-  }
-}
-__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int x, int y,
-                                            int z, unsigned long long *m) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
-      "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(m))
-      : "memory");
-}
 
 // Five consecutive raw window elements p[0..4] as floats; p is 16-byte aligned
 // for 32-bit elements and 8-byte aligned for 16-bit ones.
@@ -1476,7 +1402,7 @@ static cudaError_t launch_bp_t(const BpArgs &a, cudaStream_t s) {
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link
 // against the driver library).
-static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
+PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
   static bool tried = false;
   if (!tried) {
@@ -1533,7 +1459,7 @@ static bool tma_layout(const BpArgs &a0, bool sep, size_t budget, BpArgs *out,
   if (fixed + per_tilt > budget + 64 * 1024) return false;
   int chunk = (int)std::max<size_t>(1, (budget > fixed ? budget - fixed : 0) / per_tilt);
   chunk = std::min(chunk, std::min(kMaxChunk, a0.nt));
-  PFN_cuTensorMapEncodeTiled_v12000 enc = encode_fn();
+  PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
   if (!enc) return false;
   const cuuint64_t dims[3] = {(cuuint64_t)im.nx, (cuuint64_t)im.ny,
                               (cuuint64_t)(a0.t0 + a0.nt)};

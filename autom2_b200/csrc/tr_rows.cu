@@ -1,0 +1,837 @@
+// Back-projection and forward projection of row-invariant geometries.
+//
+// A tilt is row-invariant when its detector column does not depend on the
+// voxel row and its detector row is the voxel row plus a constant (a2 = 0,
+// b1 = b3 = 0, b2 = 1: no XTILT, no in-plane rotation, any per-tilt shift),
+// with steps |a1|, |a3| <= 1 and a1 >= 0.  Every row of the volume then
+// interpolates at the same detector columns with the same weights, so the
+// lanes of a warp run along the rows: the column walk is the same for the
+// whole warp, its cost is shared by the lane's four rows, and no two lanes
+// ever meet in a shared-memory bank.
+//
+// Stacks are kept transposed for this, [tilt][block of 128 rows][column][row]
+// ("row stacks", with `margin` columns on each side of the detector's):
+// blend_rows_kernel turns an image stack into voxel rows (the two detector
+// rows of a voxel row blended with the tilt's constant y weights), so a
+// window of columns x 128 rows is one contiguous piece, copied by a single
+// bulk copy and used without staging by the threads; unblend_rows_kernel adds
+// voxel-row sums back to detector rows.  (As boxes of a [tilt][column][row]
+// tensor, the windows arrived at 8 bytes per clock and SM and the warps
+// waited a third of the time for them.)
+//
+// The walk.  A warp owns a patch of 4 x 4 voxels in (x, z) and 128 rows, four
+// per lane.  It visits the patch's 16 voxels on a snake path whose inner axis
+// is the one with the smaller column step, so that successive voxels mostly
+// share their two detector columns, which stay in registers: EV holds the
+// even one of the two, OD the odd one.  Between the columns k and k + 1 at
+// fraction f, OD's weight is f for even k and 1 - f for odd k, which is the
+// magnitude of the coordinate modulo two columns taken as a signed Q1.31
+// word.  A step crosses at most one column boundary (steps are at most one),
+// where the register whose weight passes through zero is replaced.
+//
+// Coordinates, weights and crossings of a path are the same for all lanes, so
+// the lanes compute them side by side -- lane i position i, two tilts at a
+// time -- and leave them in shared memory as one 16-byte record per position,
+// which a step reads as a broadcast.
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+#include <stdint.h>
+
+#include <algorithm>
+
+#include "tr_device.cuh"
+#include "tr_geom.h"
+#include "tr_internal.cuh"
+
+namespace trb {
+
+namespace {
+
+constexpr int kLaneRows = 4;
+constexpr int kColBytes = kRowTile * (int)sizeof(float);  // one window column
+
+// Shared bookkeeping of one tilt for one tile: coordinate of the tile's first
+// voxel relative to kmin and the steps along x and z, Q32.32.
+struct RowTilt {
+  long long u0, sx, sz;
+  int kmin;   // detector column of window column 0
+  int flags;  // bit 0: x is the inner axis; bit 1: the window lies outside the stack
+};
+
+// FP64 setup of tilt g for the tile whose first voxel is (xc, zc) and whose
+// extents minus one are (ex, ez).
+__device__ __forceinline__ RowTilt row_tilt(const TiltGeo &g, int xc, int zc, float ox, float oz,
+                                            double ex, double ez, int pnx,
+                                            int cols) {
+  const double X = (double)((float)xc - ox), Z = (double)((float)zc - oz);
+  const double uc = g.a[0] + g.a[1] * X + g.a[3] * Z + (double)ox;
+  const double umin = floor(uc + fmin(0.0, g.a[1] * ex) + fmin(0.0, g.a[3] * ez));
+  RowTilt t;
+  t.kmin = (int)umin - 1;
+  t.u0 = __double2ll_rn((uc - (double)t.kmin) * 4294967296.0);
+  t.sx = g.A[0];
+  t.sz = g.A[2];
+  const long long m3 = t.sz < 0 ? -t.sz : t.sz;
+  t.flags = (m3 > t.sx ? 1 : 0) | (t.kmin < -cols || t.kmin > pnx ? 2 : 0);
+  t.kmin = min(max(t.kmin, -cols), pnx);
+  return t;
+}
+
+// Voxel of position i on the snake path over a 4 x 4 patch: i / 4 along the
+// outer axis, forwards and backwards in turn along the inner one.
+__host__ __device__ constexpr int snake_inner(int i) { return (i >> 2) & 1 ? 3 - (i & 3) : i & 3; }
+template <bool XIN>
+__host__ __device__ constexpr int snake_voxel(int i) {  // z * 4 + x
+  return XIN ? (i >> 2) * 4 + snake_inner(i) : snake_inner(i) * 4 + (i >> 2);
+}
+
+// Float offset of column k (>= -margin) of row block yb in a row stack of nyb
+// blocks per tilt.
+__device__ __forceinline__ size_t row_stack_at(int t, int yb, int nyb, int k, int nx, int margin) {
+  return (((size_t)t * nyb + yb) * (nx + 2 * margin) + (k + margin)) * kRowTile;
+}
+// Contiguous copies between global and shared memory (16-byte multiples): a
+// load reported to mbarrier m, and an asynchronous float addition.
+__device__ __forceinline__ void bulk_load(void *dst, const float *src, unsigned bytes,
+                                          unsigned long long *m) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+          smem_u32(dst)),
+      "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(smem_u32(m))
+      : "memory");
+}
+__device__ __forceinline__ void bulk_add(float *dst, const void *src, unsigned bytes) {
+  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(
+                   __cvta_generic_to_global(dst)),
+               "r"(smem_u32(src)), "r"(bytes)
+               : "memory");
+}
+
+// One position of a patch's path: OD's weight and a window byte offset (see
+// path_records).  Eight bytes: a broadcast read takes a wavefront per four bytes.
+struct __align__(8) PathRec {
+  float w;
+  unsigned a;
+};
+// A path: its 16 positions, the crossing positions (bit per position) at which
+// EV's and OD's column changes, and
+//   gather: the positions within [-1, nx-1], RowTilt::flags;
+//   splat: the window offsets of the last even and odd column.
+struct __align__(16) PatchPath {
+  PathRec pos[16];
+  unsigned ev, od, c, d;
+};
+
+// Paths of the patches at (px, pz) of the tile, one per half warp: lane i % 16
+// computes position i of its half's path.
+//   gather: positions 0 and 8 hold the window offset of their lower column, a
+//     crossing position that of the column to load.
+//   splat: a crossing position holds the offset of the column to add to.
+template <bool SPLAT>
+__device__ __forceinline__ void path_records(const RowTilt &tl, int px, int pz, int lane, int pnx,
+                                             PatchPath *path) {
+  const int pos = lane & 15, out = pos >> 2, in = snake_inner(pos);
+  const bool xin = tl.flags & 1;
+  const long long U = tl.u0 + (px + (xin ? in : out)) * tl.sx + (pz + (xin ? out : in)) * tl.sz;
+  const int k = (int)(U >> 32);
+  const float w = fabsf((float)(int)(unsigned)(U >> 1)) * 4.656612873077393e-10f;  // 2^-31
+  const int kp = __shfl_up_sync(0xffffffffu, k, 1);
+  const bool cross = pos > 0 && k != kp;
+  // the column that comes into reach (gather) or leaves it (splat)
+  const int col = SPLAT ? (k > kp ? kp : kp + 1) : (k > kp ? k + 1 : k);
+  const int half = lane & 16;
+  const unsigned ev = __ballot_sync(0xffffffffu, cross && !(col & 1)) >> half;
+  const unsigned od = __ballot_sync(0xffffffffu, cross && (col & 1)) >> half;
+  const unsigned in_range =
+      __ballot_sync(0xffffffffu, (unsigned)(k + tl.kmin + 1) <= (unsigned)pnx) >> half;
+  const unsigned even = (k + (k & 1)) * kColBytes, odd = (k | 1) * kColBytes;
+  const bool start = !SPLAT && (pos & 7) == 0;
+  path->pos[pos] = PathRec{w, (unsigned)(start ? k : col) * kColBytes};
+  if (pos == 15) {
+    path->ev = ev;
+    path->od = od;
+    path->c = SPLAT ? even : in_range & 0xffffu;
+    path->d = SPLAT ? odd : tl.flags;
+  }
+}
+
+__device__ __forceinline__ void lds4(f32x2 &a, f32x2 &b, unsigned addr) {
+  asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr));
+}
+
+// One tilt of a patch: win is the lane's window address.  The path is walked in
+// two halves side by side, whose loads overlap.  CHECK: positions outside
+// `valid` get nothing.
+template <bool XIN, bool CHECK>
+__device__ __forceinline__ void gather_patch(f32x2 (&acc)[16][2], unsigned win, const PatchPath *path,
+                                             unsigned mask_ev, unsigned mask_od, unsigned valid) {
+  f32x2 ev[2][2], od[2][2];
+  uint2 r[2][2];  // the records of this step and the next
+  auto fetch = [&](int j) {
+    r[j & 1][0] = *reinterpret_cast<const uint2 *>(path->pos + j);
+    r[j & 1][1] = *reinterpret_cast<const uint2 *>(path->pos + 8 + j);
+  };
+  fetch(0);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    if (j + 1 < 8) fetch(j + 1);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int i = 8 * h + j;
+      const unsigned at = win + r[j & 1][h].y;
+      if (j == 0) {
+        // the even one of columns k and k + 1, and the odd one
+        const unsigned k1 = (r[0][h].y / kColBytes & 1) * kColBytes;
+        lds4(ev[h][0], ev[h][1], at + k1);
+        lds4(od[h][0], od[h][1], at + kColBytes - k1);
+      } else {
+        asm volatile(
+            "{\n .reg .pred p, q;\n .reg .b32 t, s;\n and.b32 t, %5, %7;\n setp.ne.u32 p, t, 0;\n"
+            " and.b32 s, %6, %7;\n setp.ne.u32 q, s, 0;\n"
+            " @p ld.shared.v2.u64 {%0, %1}, [%4];\n @q ld.shared.v2.u64 {%2, %3}, [%4];\n}"
+            : "+l"(ev[h][0]), "+l"(ev[h][1]), "+l"(od[h][0]), "+l"(od[h][1])
+            : "r"(at), "r"(mask_ev), "r"(mask_od), "r"(1u << i));
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int i = 8 * h + j, v = snake_voxel<XIN>(i);
+      const float wf = __uint_as_float(r[j & 1][h].x);
+      const f32x2 w = pack2(wf, wf);
+      const f32x2 r0 = fma2(w, sub2(od[h][0], ev[h][0]), ev[h][0]);
+      const f32x2 r1 = fma2(w, sub2(od[h][1], ev[h][1]), ev[h][1]);
+      if (!CHECK || (valid >> i & 1)) {
+        acc[v][0] = add2(acc[v][0], r0);
+        acc[v][1] = add2(acc[v][1], r1);
+      }
+    }
+  }
+}
+
+// Whether quads of the view's voxels at x0, x0 + 4, ... are aligned float4s.
+__device__ __forceinline__ bool rows_vec(const VolView &v, int x0) {
+  return x0 + 3 < v.nx && ((v.sy | v.sz) & 3) == 0 && (reinterpret_cast<uintptr_t>(v.vol) & 15) == 0;
+}
+// Four voxels from p, zero where !in or beyond the row's n.
+__device__ __forceinline__ void load_quad(const float *p, bool in, bool vec, int n, float (&o)[4]) {
+  if (vec) {
+    const float4 q = in ? *reinterpret_cast<const float4 *>(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+    o[0] = q.x, o[1] = q.y, o[2] = q.z, o[3] = q.w;
+  } else {
+#pragma unroll
+    for (int x = 0; x < 4; ++x) o[x] = in && x < n ? p[x] : 0.f;
+  }
+}
+
+constexpr int kBpWarps = 8;
+constexpr int kLag = 4;  // a stage is refilled kLag tilts after its use
+constexpr int kBpX = kRowBpX, kBpZ = kRowBpZ;  // voxels of a tile along x and z
+
+// Back-projection.  Volume tile of 16 (x) x 8 (z) voxels and 128 rows; warp w
+// owns the patch at ((w % 4) 4, (w / 4) 4).  Tilts come through a ring of stages; the warps
+// take turns at filling one, which is to start the window's copy and compute
+// the eight patches' paths beside it.  (A ninth warp for this leaves 96
+// registers a thread, which spills.)
+//
+// Bound by issue and by latency at 16 warps per SM (128 registers: 64 sums):
+// 61 % of issue slots, 5.5 instructions per voxel and tilt where the general
+// kernel takes 7 with one row per table entry; shared memory 42 %, L2 17 %.
+// 1024 x 1024 x 256 voxels, 61 tilts: 3.83 ms with the row stack's 0.15 ms,
+// from 6.69 ms by the general kernel (4.3e12 from 2.4e12 voxel-tilts/s).
+template <int MODE>
+__global__ void __launch_bounds__(kBpWarps * 32, 2)
+    bp_rows_kernel(const BpArgs a, const float *__restrict__ rows, int cols, int stages) {
+  extern __shared__ __align__(128) unsigned char dsm[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int xc = blockIdx.x * kBpX, zl = blockIdx.y * kBpZ, yc = blockIdx.z * kRowTile;
+  const int nt = a.nt;
+  const unsigned win_bytes = (unsigned)cols * kColBytes;
+  const unsigned stage_bytes = win_bytes + kBpWarps * (unsigned)sizeof(PatchPath);
+  RowTilt *tt = reinterpret_cast<RowTilt *>(dsm + (size_t)stages * stage_bytes);
+  unsigned long long *full = reinterpret_cast<unsigned long long *>(tt + ((nt + 1) & ~1));
+  unsigned long long *empty = full + stages;
+
+  if (tid == 0)
+    for (int i = 0; i < stages; ++i) {
+      mbar_init(full + i, 1);
+      mbar_init(empty + i, kBpWarps);
+    }
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  for (int i = tid; i < nt; i += blockDim.x)
+    tt[i] = row_tilt(a.geo[a.t0 + i], xc, zl + a.v.zoff, a.ox, a.oz, kBpX - 1, kBpZ - 1, a.img.nx,
+                     cols);
+  __syncthreads();
+
+  const float *src = rows + row_stack_at(a.t0, blockIdx.z, gridDim.z, 0, a.img.nx, cols);
+  const size_t plane = (size_t)gridDim.z * (a.img.nx + 2 * cols) * kRowTile;
+  auto fill = [&](int t, int s) {  // by one warp: tilt t into stage s
+    unsigned char *st = dsm + (size_t)s * stage_bytes;
+    const RowTilt &tl = tt[t];
+    if (lane == 0)
+      bulk_load(st, src + (long long)(t * plane) + (long long)tl.kmin * kRowTile, win_bytes,
+                full + s);
+    PatchPath *paths = reinterpret_cast<PatchPath *>(st + win_bytes);
+#pragma unroll 1
+    for (int b = 0; b < kBpWarps / 2; ++b) {
+      const int w = 2 * b + (lane >> 4);
+      path_records<false>(tl, (w & 3) * 4, (w >> 2) * 4, lane, a.img.nx, paths + w);
+    }
+    __syncwarp();
+    if (lane == 0) mbar_expect_tx(full + s, win_bytes);  // the stage's one arrival
+  };
+  for (int t = warp; t < min(stages - kLag, nt); t += kBpWarps) fill(t, t);
+
+  // The tile's voxels are read at the end: into L2 meanwhile, one 64-byte
+  // segment (a section's 16 x) per row and section.
+  for (int i = tid; i < kRowTile * kBpZ; i += kBpWarps * 32) {
+    const int y = yc + i / kBpZ, z = zl + i % kBpZ;
+    if (y < a.v.ny && z < a.v.nz)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(a.v.vol + (size_t)y * a.v.sy +
+                                                     (size_t)z * a.v.sz + xc));
+  }
+  f32x2 acc[16][2];
+#pragma unroll
+  for (int v = 0; v < 16; ++v) acc[v][0] = acc[v][1] = 0ull;
+
+  bool ok = true;
+  int s = 0;            // stage of tilt t, and the parity of its use
+  unsigned parity = 0;
+  for (int t = 0; t < nt; ++t) {
+    if ((t & (kBpWarps - 1)) == warp && t + stages - kLag < nt) {
+      // the stage of tilt t - kLag, which the slowest warp has left or is about to
+      const int s2 = s >= kLag ? s - kLag : s - kLag + stages;
+      if (t >= kLag)
+        ok = mbar_wait_bounded(empty + s2, s >= kLag ? parity : parity ^ 1u, 1ll << 31, a.err);
+      ok = __all_sync(0xffffffffu, ok);
+      if (ok) fill(t + stages - kLag, s2);
+    }
+    ok = ok && mbar_wait_bounded(full + s, parity, 1ll << 31, a.err);
+    if (!__all_sync(0xffffffffu, ok)) {
+      ok = false;
+      break;
+    }
+    const unsigned char *st = dsm + (size_t)s * stage_bytes;
+    const PatchPath *path = reinterpret_cast<const PatchPath *>(st + win_bytes) + warp;
+    const unsigned win = smem_u32(st) + lane * (kLaneRows * 4);
+    const uint4 m = *reinterpret_cast<const uint4 *>(&path->ev);  // ev, od, in range, flags
+    if (m.w & 2) {
+      // nothing of the stack in reach
+    } else if (MODE == BP_NORM && m.z != 0xffffu) {
+      if (m.w & 1) gather_patch<true, true>(acc, win, path, m.x, m.y, m.z);
+      else gather_patch<false, true>(acc, win, path, m.x, m.y, m.z);
+    } else {
+      if (m.w & 1) gather_patch<true, false>(acc, win, path, m.x, m.y, m.z);
+      else gather_patch<false, false>(acc, win, path, m.x, m.y, m.z);
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(empty + s);
+    if (++s == stages) s = 0, parity ^= 1u;
+  }
+  if (__syncthreads_or(!ok)) {
+    // Report, give the copies in flight a bounded chance to land, and leave the
+    // tile's voxels untouched.
+    if (!ok && lane == 0) {
+      atomicExch(a.err, 1);
+      atomicExch(a.err + 1, 1);
+      for (int i = 0; i < stages; ++i)
+        for (unsigned p = 0; p < 2; ++p) mbar_wait_bounded(full + i, p, 1ll << 24, nullptr);
+    }
+    return;
+  }
+
+  // Epilogue.  The sums go through shared memory, [row][section][16 x] with
+  // the 16-byte pieces of a row exchanged so that neither side meets in a
+  // bank, and the volume is read and written by sections' rows of 64 bytes.
+  float4 *sum = reinterpret_cast<float4 *>(dsm);  // [128][32]
+  {
+    const int px = warp & 3, pz = (warp >> 2) * 4;
+#pragma unroll
+    for (int r = 0; r < kLaneRows; ++r)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        float f[4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          float lo, hi;
+          unpack2(acc[k * 4 + x][r >> 1], lo, hi);
+          f[x] = r & 1 ? hi : lo;
+        }
+        sum[(lane * 4 + r) * 32 + (((pz + k) * 4 + px) ^ (lane & 7))] =
+            make_float4(f[0], f[1], f[2], f[3]);
+      }
+  }
+  __syncthreads();
+  const int x0 = xc + (lane & 3) * 4, z = zl + (lane >> 2);
+  const bool inz = z < a.v.nz && x0 < a.v.nx;
+  const bool vec = rows_vec(a.v, x0);
+  const int gx = (a.v.nx + kTX - 1) / kTX, gy = (a.v.ny + kTY - 1) / kTY;
+  constexpr int kBatch = 8;  // rows whose reads are in flight together
+#pragma unroll 1
+  for (int i0 = 0; i0 < kRowTile / kBpWarps; i0 += kBatch) {
+    float old[kBatch][4], scale[kBatch];
+    int slot[kBatch];
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      const int y = yc + warp * (kRowTile / kBpWarps) + i0 + i;
+      const bool in = inz && y < a.v.ny;
+      load_quad(a.v.vol + (size_t)y * a.v.sy + (size_t)z * a.v.sz + x0, in, vec, a.v.nx - x0,
+                old[i]);
+      scale[i] = 1.f;
+      slot[i] = -1;
+      if (MODE == BP_SIRT && in) {
+        slot[i] = __ldg(a.wslot + ((size_t)(z / kTZ) * gy + y / kTY) * gx + x0 / kTX);
+        if (a.wrow) scale[i] = __ldg(a.wrow + y);  // interior tiles: one weight per row
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      const int row = warp * (kRowTile / kBpWarps) + i0 + i, y = yc + row;
+      if (!inz || y >= a.v.ny) continue;
+      const float4 q = sum[row * 32 + (lane ^ ((row >> 2) & 7))];
+      const float s[4] = {q.x, q.y, q.z, q.w};
+      const float sc = MODE == BP_SIRT ? (scale[i] != 0.f ? a.gamma / scale[i] : 0.f) : a.gamma;
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        if (MODE == BP_SIRT && slot[i] >= 0) {
+          // voxel of the border tile's compact weights (BpArgs::wslot)
+          const float w = x0 + x < a.v.nx
+                              ? a.wtvol[(size_t)slot[i] * kTileVox +
+                                        ((z % kTZ) * kTY + y % kTY) * kTX + (x0 + x) % kTX]
+                              : 0.f;
+          if (w != 0.f) old[i][x] += s[x] * (a.gamma / w);
+        } else {
+          old[i][x] += s[x] * sc;
+        }
+      }
+      float *p = a.v.vol + (size_t)y * a.v.sy + (size_t)z * a.v.sz + x0;
+      if (vec) {
+        *reinterpret_cast<float4 *>(p) = make_float4(old[i][0], old[i][1], old[i][2], old[i][3]);
+      } else {
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+          if (x0 + x < a.v.nx) p[x] = old[i][x];
+      }
+    }
+  }
+}
+
+// ------------------------------------------------------------ forward
+
+// Adds the lane's four rows r to window column `addr`.
+__device__ __forceinline__ void add_col(unsigned addr, f32x2 r0, f32x2 r1) {
+  f32x2 a, b;
+  lds4(a, b, addr);
+  a = add2(a, r0);
+  b = add2(b, r1);
+  asm volatile("st.shared.v2.u64 [%0], {%1, %2};" ::"r"(addr), "l"(a), "l"(b));
+}
+
+// One tilt of a patch's splat; win: the lane's window address.  Two running
+// sums take the place of EV and OD: all = EV + OD and od = OD, one addition
+// and one fused multiply-add per voxel pair from the record's one weight.  At
+// a crossing one register goes to its column; the column's rows are read a
+// position ahead (successive crossings never add to the same column), and the
+// rest is a real branch (the masks are the same for the whole warp), since
+// predicated instructions would be issued at every position.
+template <bool XIN>
+__device__ __forceinline__ void splat_patch(const f32x2 (&vox)[16][2], unsigned win,
+                                            const PatchPath *path) {
+  const uint4 m = *reinterpret_cast<const uint4 *>(&path->ev);  // ev, od, last columns
+  const unsigned cross = m.x | m.y;
+  f32x2 all0 = 0ull, all1 = 0ull, od0 = 0ull, od1 = 0ull;
+  f32x2 c0 = 0ull, c1 = 0ull;  // rows of the column of the next crossing
+  uint2 q[3];
+  q[0] = *reinterpret_cast<const uint2 *>(path->pos);
+  q[1] = *reinterpret_cast<const uint2 *>(path->pos + 1);
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    if (i + 2 < 16) q[(i + 2) % 3] = *reinterpret_cast<const uint2 *>(path->pos + i + 2);
+    if (i > 0)
+      asm volatile(
+          "{\n .reg .pred p, q;\n .reg .b32 t, s;\n .reg .b64 c, d;\n"
+          " and.b32 t, %7, %9;\n setp.eq.u32 p, t, 0;\n @p bra.uni DONE;\n"
+          " and.b32 s, %8, %9;\n setp.eq.u32 q, s, 0;\n"
+          " sub.rn.f32x2 c, %0, %2;\n sub.rn.f32x2 d, %1, %3;\n @q bra.uni ODD;\n"
+          " add.rn.f32x2 c, %4, c;\n add.rn.f32x2 d, %5, d;\n"
+          " st.shared.v2.u64 [%6], {c, d};\n mov.b64 %0, %2;\n mov.b64 %1, %3;\n bra.uni DONE;\n"
+          "ODD:\n mov.b64 %0, c;\n mov.b64 %1, d;\n add.rn.f32x2 c, %4, %2;\n"
+          " add.rn.f32x2 d, %5, %3;\n st.shared.v2.u64 [%6], {c, d};\n mov.b64 %2, 0;\n"
+          " mov.b64 %3, 0;\n"
+          "DONE:\n}"
+          : "+l"(all0), "+l"(all1), "+l"(od0), "+l"(od1)
+          : "l"(c0), "l"(c1), "r"(win + q[i % 3].y), "r"(cross), "r"(m.x), "r"(1u << i));
+    if (i + 1 < 16)
+      asm volatile(
+          "{\n .reg .pred p;\n .reg .b32 t;\n and.b32 t, %3, %4;\n setp.ne.u32 p, t, 0;\n"
+          " @p ld.shared.v2.u64 {%0, %1}, [%2];\n}"
+          : "+l"(c0), "+l"(c1)
+          : "r"(win + q[(i + 1) % 3].y), "r"(cross), "r"(2u << i));
+    const int v = snake_voxel<XIN>(i);
+    const float wf = __uint_as_float(q[i % 3].x);
+    const f32x2 w = pack2(wf, wf);
+    all0 = add2(all0, vox[v][0]);
+    all1 = add2(all1, vox[v][1]);
+    od0 = fma2(w, vox[v][0], od0);
+    od1 = fma2(w, vox[v][1], od1);
+  }
+  add_col(win + m.z, sub2(all0, od0), sub2(all1, od1));
+  add_col(win + m.w, od0, od1);
+}
+
+constexpr int kFpWarps = 8;
+constexpr int kFpX = kRowFpX, kFpZ = kRowFpZ;
+
+// Forward projection of a tile of 16 (x) x 8 (z) voxels and 128 rows into the
+// row stack.  The voxels stay in registers.  The tilts' windows stand in a
+// ring of slots and go from warp to warp: warp w adds its patch to a tilt's
+// window once warp w - 1 has, so that no two add to it at a time and the
+// additions need no atomics; the last warp sends the finished window out as one
+// bulk reduction and hands the slot back to the first.  (With all warps in step
+// over eight windows at a time, barriers and the wait for the reductions took a
+// quarter of the time.)
+//
+// Bound as the back-projection, with more instructions (7 per voxel and tilt):
+// a column that leaves the path is a read, an addition and a write of its
+// window.  1024 x 1024 x 256 voxels, 61 tilts: 6.07 ms with the row sums'
+// conversion, from 8.12 ms by the general splat, whose 32-bit fixed point this
+// replaces by float sums.
+__global__ void __launch_bounds__(kFpWarps * 32, 2)
+    fp_rows_kernel(const FpArgs a, float *__restrict__ rows, int cols, int slots, int ahead) {
+  extern __shared__ __align__(128) unsigned char dsm[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int xc = blockIdx.x * kFpX, zl = blockIdx.y * kFpZ, yc = blockIdx.z * kRowTile;
+  const int nt = a.nt;
+  const unsigned win_bytes = (unsigned)cols * kColBytes;
+  // the windows' room also holds the tile's voxels at first
+  RowTilt *tt = reinterpret_cast<RowTilt *>(dsm + max(slots * win_bytes, (unsigned)kRowTile * 512));
+  PatchPath *paths = reinterpret_cast<PatchPath *>(tt + ((nt + 1) & ~1)) + warp * 2;
+  // per slot: warp w < 7 has added to it; [7]: it may be used again
+  unsigned long long *hand = reinterpret_cast<unsigned long long *>(
+      reinterpret_cast<PatchPath *>(tt + ((nt + 1) & ~1)) + kFpWarps * 2);
+  for (int i = tid; i < slots * kFpWarps; i += blockDim.x) mbar_init(hand + i, 1);
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  for (int i = tid; i < nt; i += blockDim.x)
+    tt[i] = row_tilt(a.geo[a.t0 + i], xc, zl + a.v.zoff, a.ox, a.oz, kFpX - 1, kFpZ - 1, a.pnx, cols);
+
+  // The tile's voxels, read by sections' rows of 64 bytes, through shared memory
+  // (the windows') to the lanes that own their rows, as in the back-projection.
+  f32x2 vox[16][2];
+  bool any = a.v.vol == nullptr;
+  if (a.v.vol) {
+    float4 *buf = reinterpret_cast<float4 *>(dsm);  // [128][32]
+    const int x0 = xc + (lane & 3) * 4, z = zl + (lane >> 2);
+    const bool inz = z < a.v.nz, vec = rows_vec(a.v, x0);
+#pragma unroll 8
+    for (int i = 0; i < kRowTile / kFpWarps; ++i) {
+      const int row = warp * (kRowTile / kFpWarps) + i, y = yc + row;
+      float f[4];
+      load_quad(a.v.vol + (size_t)y * a.v.sy + (size_t)z * a.v.sz + x0, inz && y < a.v.ny, vec,
+                a.v.nx - x0, f);
+      buf[row * 32 + (lane ^ ((row >> 2) & 7))] = make_float4(f[0], f[1], f[2], f[3]);
+      any |= f[0] != 0.f || f[1] != 0.f || f[2] != 0.f || f[3] != 0.f;
+    }
+  }
+  if (!__syncthreads_or(any)) return;  // an all-zero tile adds nothing
+  {
+    const int px = warp & 3, pz = (warp >> 2) * 4;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float4 f[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        if (a.v.vol) {
+          f[r] = reinterpret_cast<const float4 *>(
+              dsm)[(lane * 4 + r) * 32 + (((pz + k) * 4 + px) ^ (lane & 7))];
+        } else {
+          const int x0 = xc + px * 4;
+          const bool in = yc + lane * 4 + r < a.v.ny && zl + pz + k < a.v.nz;
+          f[r] = make_float4(in && x0 < a.v.nx ? 1.f : 0.f, in && x0 + 1 < a.v.nx ? 1.f : 0.f,
+                             in && x0 + 2 < a.v.nx ? 1.f : 0.f, in && x0 + 3 < a.v.nx ? 1.f : 0.f);
+        }
+      }
+      vox[k * 4 + 0][0] = pack2(f[0].x, f[1].x), vox[k * 4 + 0][1] = pack2(f[2].x, f[3].x);
+      vox[k * 4 + 1][0] = pack2(f[0].y, f[1].y), vox[k * 4 + 1][1] = pack2(f[2].y, f[3].y);
+      vox[k * 4 + 2][0] = pack2(f[0].z, f[1].z), vox[k * 4 + 2][1] = pack2(f[2].z, f[3].z);
+      vox[k * 4 + 3][0] = pack2(f[0].w, f[1].w), vox[k * 4 + 3][1] = pack2(f[2].w, f[3].w);
+    }
+  }
+  __syncthreads();
+
+  if (a.v.vol) {
+    // Into L2: the voxels of the tile that takes this one's place on the SM.
+    unsigned n = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x + ahead;
+    const unsigned bx = n % gridDim.x, by = n / gridDim.x % gridDim.y, bz = n / gridDim.x / gridDim.y;
+    for (int i = tid; i < kRowTile * kFpZ; i += blockDim.x) {
+      const int y = bz * kRowTile + i / kFpZ, z = by * kFpZ + i % kFpZ;
+      if (y < a.v.ny && z < a.v.nz)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(a.v.vol + (size_t)y * a.v.sy +
+                                                       (size_t)z * a.v.sz + bx * kFpX));
+    }
+  }
+
+  float *dst = rows + row_stack_at(a.t0, blockIdx.z, gridDim.z, 0, a.pnx, cols);
+  const size_t plane = (size_t)gridDim.z * (a.pnx + 2 * cols) * kRowTile;
+  bool ok = true;
+  int s = 0;             // slot of tilt t, and the parity of its use
+  unsigned parity = 0;
+  for (int t = 0; t < nt; ++t) {
+    if (!(t & 1)) {  // this warp's paths of two tilts
+      __syncwarp();
+      path_records<true>(tt[min(t + (lane >> 4), nt - 1)], (warp & 3) * 4, (warp >> 2) * 4, lane,
+                         a.pnx, paths + (lane >> 4));
+      __syncwarp();
+    }
+    unsigned char *win = dsm + (size_t)s * win_bytes;
+    unsigned long long *h = hand + s * kFpWarps;
+    if (warp > 0) {
+      ok = mbar_wait_bounded(h + warp - 1, parity, 1ll << 31, a.err);
+    } else {
+      if (t >= slots) ok = mbar_wait_bounded(h + kFpWarps - 1, parity ^ 1u, 1ll << 31, a.err);
+      if (ok)
+        for (unsigned e = lane; e < win_bytes / 16; e += 32)
+          reinterpret_cast<float4 *>(win)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+      __syncwarp();
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) break;
+    const RowTilt &tl = tt[t];
+    const unsigned at = smem_u32(win) + lane * (kLaneRows * 4);
+    if (tl.flags & 1) splat_patch<true>(vox, at, paths + (t & 1));
+    else splat_patch<false>(vox, at, paths + (t & 1));
+    __syncwarp();
+    if (lane == 0) {
+      if (warp < kFpWarps - 1) {
+        mbar_arrive(h + warp);
+      } else {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        if (!(tl.flags & 2))
+          bulk_add(dst + (long long)(t * plane) + (long long)tl.kmin * kRowTile, win, win_bytes);
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        // the reduction before this one has read its slot
+        asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        if (t > 0) mbar_arrive(hand + (s > 0 ? s : slots) * kFpWarps - 1);
+      }
+    }
+    if (++s == slots) s = 0, parity ^= 1u;
+  }
+  if (!ok && lane == 0 && a.err) {  // report; the sums of this tile are incomplete
+    atomicExch(a.err, 1);
+    atomicExch(a.err + 1, 1);
+  }
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
+
+// ------------------------------------------------------------ row stacks
+
+template <typename IT>
+__device__ __forceinline__ float img_f(const IT *p, size_t i);
+template <>
+__device__ __forceinline__ float img_f<float>(const float *p, size_t i) { return __ldg(p + i); }
+template <>
+__device__ __forceinline__ float img_f<__half>(const __half *p, size_t i) {
+  return __half2float(p[i]);
+}
+template <>
+__device__ __forceinline__ float img_f<__nv_bfloat16>(const __nv_bfloat16 *p, size_t i) {
+  return __bfloat162float(p[i]);
+}
+
+// Lower detector row of voxel row y and the upper one's weight, as the
+// reference evaluates them (b1 = b3 = 0, b2 = 1).
+__device__ __forceinline__ int voxel_row(const TiltGeo &g, int y, float oy, float &dy) {
+  const double v = g.b[0] + g.b[2] * (double)((float)y - oy) + (double)oy;
+  const int y0 = (int)floor(v);
+  dy = (float)(v - (double)y0);
+  return y0;
+}
+
+constexpr int kBlendCols = 32, kBlendRows = 64;
+
+// Image stack -> row stack: the blended value of voxel row y at detector column
+// k.  NORM: columns -1..nx of the edge-clamped image, rows normalised by their
+// in-image weight (zero where neither row is inside); else columns 0..nx-1,
+// in-image rows only.  Zero in the other margin columns and below the volume.
+template <bool NORM, typename IT>
+__global__ void __launch_bounds__(256)
+    blend_rows_kernel(const ImgView im, const TiltGeo *__restrict__ geo, int t0, float oy, int vny,
+                      int margin, float *__restrict__ out) {
+  __shared__ float s[kBlendCols][kBlendRows + 1];
+  const int t = blockIdx.z, c0 = blockIdx.x * kBlendCols, r0 = blockIdx.y * kBlendRows;
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, tc = im.nx + 2 * margin;
+  const TiltGeo &g = geo[t0 + t];
+  const IT *p = reinterpret_cast<const IT *>(im.p) + (size_t)(t0 + t) * im.tstride;
+  const float sc = im.scale ? im.scale[t0 + t] : 1.f;
+  int k = c0 + lane - margin;
+  const bool ink = NORM ? k >= -1 && k <= im.nx : k >= 0 && k < im.nx;
+  k = min(max(k, 0), im.nx - 1);
+#pragma unroll
+  for (int i = 0; i < kBlendRows / 8; ++i) {
+    const int r = wp + 8 * i, y = r0 + r;
+    float v = 0.f;
+    if (ink && y < vny) {
+      float dy;
+      const int y0 = voxel_row(g, y, oy, dy);
+      const float w0 = (y0 >= 0 && y0 < im.ny) ? 1 - dy : 0.f;
+      const float w1 = (y0 + 1 >= 0 && y0 + 1 < im.ny) ? dy : 0.f;
+      const float p0 = w0 != 0.f ? img_f(p, (size_t)y0 * im.nx + k) * sc : 0.f;
+      const float p1 = w1 != 0.f ? img_f(p, (size_t)(y0 + 1) * im.nx + k) * sc : 0.f;
+      v = w0 * p0 + w1 * p1;
+      if (NORM) v = w0 + w1 != 0.f ? v / (w0 + w1) : 0.f;
+    }
+    s[lane][r] = v;
+  }
+  __syncthreads();
+  float *o = out + ((size_t)(t0 + t) * ((vny + kRowTile - 1) / kRowTile) + r0 / kRowTile) * tc * kRowTile +
+             r0 % kRowTile + lane;
+#pragma unroll
+  for (int i = 0; i < kBlendCols / 8; ++i) {
+    const int c = wp + 8 * i;
+    if (c0 + c >= tc) break;
+#pragma unroll
+    for (int h = 0; h < kBlendRows / 32; ++h)
+      o[(size_t)(c0 + c) * kRowTile + 32 * h] = s[c][lane + 32 * h];
+  }
+}
+
+// Row stack -> image stack: val[t][j][k] += the voxel-row sums that splat onto
+// detector row j, (1 - dy) of the row whose lower detector row is j and dy of
+// the one below.
+__global__ void __launch_bounds__(256)
+    unblend_rows_kernel(const float *__restrict__ rows, const TiltGeo *__restrict__ geo, int t0,
+                        float oy, int vny, int margin, float *__restrict__ val, long long tstride,
+                        int nx, int ny) {
+  constexpr int kHalo = 3;  // voxel rows j - S - 2 .. j - S + 1, S = floor(b0)
+  __shared__ float s[kBlendCols][kBlendRows + kHalo + 2];
+  __shared__ int sy0[kBlendRows + kHalo];
+  __shared__ float sdy[kBlendRows + kHalo];
+  const int t = blockIdx.z, c0 = blockIdx.x * kBlendCols, j0 = blockIdx.y * kBlendRows;
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const TiltGeo &g = geo[t0 + t];
+  const int tc = nx + 2 * margin, nyb = (vny + kRowTile - 1) / kRowTile;
+  const int y0 = j0 - (int)floor(g.b[0]) - 2;  // first voxel row of the tile
+  if (threadIdx.x < kBlendRows + kHalo) {
+    float dy;
+    sy0[threadIdx.x] = voxel_row(g, y0 + threadIdx.x, oy, dy);
+    sdy[threadIdx.x] = dy;
+  }
+  for (int c = wp; c < kBlendCols; c += 8)
+    for (int r = lane; r < kBlendRows + kHalo; r += 32) {
+      const int y = y0 + r, k = c0 + c;
+      s[c][r] = k < nx && y >= 0 && y < vny
+                    ? __ldg(rows + (((size_t)(t0 + t) * nyb + y / kRowTile) * tc + k + margin) *
+                                       kRowTile + y % kRowTile)
+                    : 0.f;
+    }
+  __syncthreads();
+  const int k = c0 + lane;
+  if (k >= nx) return;
+#pragma unroll
+  for (int i = 0; i < kBlendRows / 8; ++i) {
+    const int r = wp + 8 * i, j = j0 + r;
+    if (j >= ny) break;
+    float v = 0.f;
+#pragma unroll
+    for (int h = 0; h <= kHalo; ++h) {
+      const int q = r + h;
+      if (sy0[q] == j) v += (1 - sdy[q]) * s[lane][q];
+      else if (sy0[q] == j - 1) v += sdy[q] * s[lane][q];
+    }
+    if (v != 0.f) {
+      float *o = val + (size_t)(t0 + t) * tstride + (size_t)j * nx + k;
+      *o += v;
+    }
+  }
+}
+
+}  // namespace
+
+// ------------------------------------------------------------ launchers
+
+cudaError_t launch_blend_rows(const ImgView &im, const TiltGeo *geo, int t0, int nt, float oy,
+                              int vny, int margin, bool norm, float *rows, cudaStream_t s) {
+  const int tc = im.nx + 2 * margin;
+  const dim3 grid((tc + kBlendCols - 1) / kBlendCols,
+                  (vny + kRowTile - 1) / kRowTile * (kRowTile / kBlendRows), nt);
+  auto go = [&](auto *tag) {
+    using IT = std::remove_pointer_t<decltype(tag)>;
+    if (norm)
+      blend_rows_kernel<true, IT><<<grid, 256, 0, s>>>(im, geo, t0, oy, vny, margin, rows);
+    else
+      blend_rows_kernel<false, IT><<<grid, 256, 0, s>>>(im, geo, t0, oy, vny, margin, rows);
+  };
+  if (im.dtype == IMG_F16) go((__half *)nullptr);
+  else if (im.dtype == IMG_BF16) go((__nv_bfloat16 *)nullptr);
+  else go((float *)nullptr);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_unblend_rows(const float *rows, const TiltGeo *geo, int t0, int nt, float oy,
+                                int vny, int margin, float *val, long long tstride, int nx, int ny,
+                                cudaStream_t s) {
+  const dim3 grid((nx + kBlendCols - 1) / kBlendCols, (ny + kBlendRows - 1) / kBlendRows, nt);
+  unblend_rows_kernel<<<grid, 256, 0, s>>>(rows, geo, t0, oy, vny, margin, val, tstride, nx, ny);
+  return cudaGetLastError();
+}
+
+// Dynamic shared memory of the kernels.
+static size_t bp_rows_smem(int cols, int nt, int stages) {
+  return (size_t)stages * (cols * kColBytes + kBpWarps * sizeof(PatchPath) + 16) +
+         (size_t)((nt + 1) & ~1) * sizeof(RowTilt);  // at least kRowTile * 512 for the epilogue
+}
+static int bp_rows_stages(int cols, int nt) {
+  const size_t fixed = bp_rows_smem(cols, nt, 0), per = bp_rows_smem(cols, 0, 1);
+  if (fixed >= kRowSmem) return 0;
+  // two CTAs per SM when that leaves windows in flight
+  if (fixed < kRowSmem2 && (kRowSmem2 - fixed) / per >= kLag + 2)
+    return (int)std::min<size_t>(10, (kRowSmem2 - fixed) / per);
+  return (int)std::min<size_t>(10, (kRowSmem - fixed) / per);
+}
+bool bp_rows_fits(int cols, int nt) { return bp_rows_stages(cols, nt) >= kLag + 2; }
+
+static size_t fp_rows_smem(int cols, int nt, int slots) {
+  return std::max<size_t>((size_t)slots * cols * kColBytes, kRowTile * 512) +
+         (size_t)((nt + 1) & ~1) * sizeof(RowTilt) + kFpWarps * 2 * sizeof(PatchPath) +
+         slots * kFpWarps * sizeof(unsigned long long);
+}
+// Slots: eight are in the warps' hands, one is being sent out.
+static int fp_rows_slots(int cols, int nt) {
+  for (size_t room : {kRowSmem2, kRowSmem})
+    for (int n = 11; n >= 9; --n)
+      if (fp_rows_smem(cols, nt, n) <= room) return n;
+  return 0;
+}
+bool fp_rows_fits(int cols, int nt) { return fp_rows_slots(cols, nt) > 0; }
+
+template <int MODE>
+static cudaError_t launch_bp_rows_t(const BpArgs &a, const float *rows, int cols, cudaStream_t s) {
+  const int stages = bp_rows_stages(cols, a.nt);
+  const size_t smem = std::max<size_t>(bp_rows_smem(cols, a.nt, stages), kRowTile * 512);
+  cudaError_t e = cudaFuncSetAttribute(bp_rows_kernel<MODE>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const dim3 grid((a.v.nx + kBpX - 1) / kBpX, (a.v.nz + kBpZ - 1) / kBpZ,
+                  (a.v.ny + kRowTile - 1) / kRowTile);
+  bp_rows_kernel<MODE><<<grid, kBpWarps * 32, smem, s>>>(a, rows, cols, stages);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_bp_rows(int mode, const BpArgs &a, const float *rows, int cols, cudaStream_t s) {
+  if (mode == BP_NORM) return launch_bp_rows_t<BP_NORM>(a, rows, cols, s);
+  if (mode == BP_SIRT) return launch_bp_rows_t<BP_SIRT>(a, rows, cols, s);
+  return launch_bp_rows_t<BP_SUM>(a, rows, cols, s);
+}
+
+cudaError_t launch_fp_rows(const FpArgs &a, float *rows, int cols, int nsm, cudaStream_t s) {
+  const int slots = fp_rows_slots(cols, a.nt);
+  const size_t smem = fp_rows_smem(cols, a.nt, slots);
+  cudaError_t e = cudaFuncSetAttribute(fp_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)smem);
+  if (e != cudaSuccess) return e;
+  const dim3 grid((a.v.nx + kFpX - 1) / kFpX, (a.v.nz + kFpZ - 1) / kFpZ,
+                  (a.v.ny + kRowTile - 1) / kRowTile);
+  fp_rows_kernel<<<grid, kFpWarps * 32, smem, s>>>(a, rows, cols, slots, smem <= kRowSmem2 ? 2 * nsm : nsm);
+  return cudaGetLastError();
+}
+
+}  // namespace trb
