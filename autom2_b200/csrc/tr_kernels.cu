@@ -333,22 +333,47 @@ __device__ __forceinline__ void bp_epilogue(const BpArgs &a, const float (&acc)[
   // Voxel k of this thread in a tile's compact weights.
   const int local0 = (((threadIdx.x >> 5) / kTY) * kNV * kTY + (threadIdx.x >> 5) % kTY) * kTX +
                      (threadIdx.x & 31);
+  // A break per section would chain each section's read to the write before it;
+  // here eight reads are in flight together.  General geometry, 1024 x 1024:
+  // x 64 voxels, 1 tilt 332 -> 168 us, 8 tilts 550 -> 470 us; x 256, 61 tilts
+  // 11.67 -> 11.55 ms.
+  const size_t idx0 = (size_t)y * a.v.sy + (size_t)zbase * a.v.sz + x;
+  const int nk = a.v.nz - zbase;  // sections k < nk exist
+  if (MODE == BP_WEIGHTS) {
 #pragma unroll
-  for (int k = 0; k < kNV; ++k) {
-    const int z = zbase + k;
-    if (z >= a.v.nz) break;
-    const size_t idx = (size_t)y * a.v.sy + (size_t)z * a.v.sz + x;
-    const size_t cidx = (size_t)slot * kTileVox + local0 + k * (kTY * kTX);
-    if (MODE == BP_NORM || MODE == BP_SUM) {
-      a.v.vol[idx] += a.gamma * acc[k];
-    } else if (MODE == BP_SIRT) {
-      float w;
-      if (!a.wslot) w = a.wtvol[idx];
-      else if (slot < 0) w = SEP ? a.wrow[y] : a.wfull;
-      else w = a.wtvol[cidx];
-      if (w != 0.f) a.v.vol[idx] += acc[k] / w * a.gamma;
-    } else {
-      a.out[a.wslot ? cidx : idx] = acc[k];
+    for (int k = 0; k < kNV; ++k)
+      if (k < nk)
+        a.out[a.wslot ? (size_t)slot * kTileVox + local0 + k * (kTY * kTX)
+                      : idx0 + (size_t)k * a.v.sz] = acc[k];
+    return;
+  }
+  float wrow = 0.f;
+  if (MODE == BP_SIRT && a.wslot && slot < 0) wrow = SEP ? a.wrow[y] : a.wfull;
+  constexpr int kBatch = 8;
+#pragma unroll
+  for (int k0 = 0; k0 < kNV; k0 += kBatch) {
+    float old[kBatch], w[kBatch];
+#pragma unroll
+    for (int h = 0; h < kBatch; ++h) {
+      const int k = k0 + h;
+      const size_t idx = idx0 + (size_t)k * a.v.sz;
+      old[h] = k < nk ? a.v.vol[idx] : 0.f;
+      if (MODE == BP_SIRT) {
+        w[h] = wrow;
+        if (k < nk && !a.wslot) w[h] = a.wtvol[idx];
+        else if (k < nk && slot >= 0)
+          w[h] = a.wtvol[(size_t)slot * kTileVox + local0 + k * (kTY * kTX)];
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < kBatch; ++h) {
+      const int k = k0 + h;
+      if (k >= nk) continue;
+      if (MODE == BP_SIRT) {
+        if (w[h] != 0.f) a.v.vol[idx0 + (size_t)k * a.v.sz] = old[h] + acc[k] / w[h] * a.gamma;
+      } else {
+        a.v.vol[idx0 + (size_t)k * a.v.sz] = old[h] + a.gamma * acc[k];
+      }
     }
   }
 }
