@@ -293,43 +293,105 @@ cudaError_t launch_rweight(const FilterArgs &f, cudaStream_t s) {
 // evaluated here as a direct sum in double precision (251 products per
 // output; the kernel's many small taps make float accumulation lose ~1e-6).
 // One CTA per row: the row's extended samples e[t] = x[(t - 124) mod L],
-// t in [0, nx + 250], and the taps live in shared memory.
+// t in [0, nx + 250], and the taps live in shared memory in double.
+//
+// Bound by FP64 (one fused multiply-add per tap and sample: 0.31 ms for 22.9 M
+// samples).  A thread takes eight consecutive outputs and slides a window of
+// eight samples over the taps, so that a tap costs it two shared reads and
+// eight multiply-adds; a thread's segment starts on its own pair of banks (nine
+// doubles apart).  61 x 523 rows of 717: 1.42 -> 0.51 ms (one output per thread:
+// two reads, a conversion and a multiply-add per tap).
 
 constexpr int kFbpTaps = 251;
+constexpr int kFbpRun = 8;  // outputs of a thread
+// Shared slot of sample t: one pad entry after every kFbpRun.
+__host__ __device__ __forceinline__ int fbp_slot(int t) { return t + t / kFbpRun; }
 
-__global__ void __launch_bounds__(256) fbp_filter_kernel(float *rows, int nx, int L, int mode) {
-  extern __shared__ double fsm[];
-  double *f = fsm;                                     // [251]
-  float *e = reinterpret_cast<float *>(fsm + kFbpTaps);  // [nx + 250]
+// The taps, formed in the reference's precision (:137-178), on the host: their
+// divisions would cost a CTA more than staging its row.
+struct FbpTaps {
+  float f[kFbpTaps];
+};
+float fbp_tap(int k, int mode) {
+  const double pi = 3.14159265358979323846;
   const int half = kFbpTaps / 2;
-  for (int k = threadIdx.x; k < kFbpTaps; k += blockDim.x) {
-    // The reference's kernels, formed in the same precision (:137-178).
-    const double pi = 3.14159265358979323846;
-    float v;
-    if (mode == 1) {
-      const int n = k - half;
-      v = n == 0 ? (float)(pi / 4) : ((n % 2) != 0 ? (float)(-1.0 / (pi * n * n)) : 0.f);
-    } else {
-      const double n = (double)((float)(k - half));
-      v = (float)(-2.0 / (pi * (4.0 * n * n - 1.0)));
-    }
-    f[k] = (double)v;
+  if (mode == 1) {
+    const int n = k - half;
+    return n == 0 ? (float)(pi / 4) : ((n % 2) != 0 ? (float)(-1.0 / (pi * n * n)) : 0.f);
   }
-  float *r = rows + (size_t)blockIdx.x * nx;
+  const double n = (double)((float)(k - half));
+  return (float)(-2.0 / (pi * (4.0 * n * n - 1.0)));
+}
+// Sample e[t] of the padded, extended row r, t in [0, nx + 250).
+__device__ __forceinline__ float fbp_sample(const float *r, int t, int nx, int L) {
   const int np = nx + 2;
   const int end = np >= L - np ? L : 2 * np;  // mirrored extension, zeros after
-  for (int t = threadIdx.x; t < nx + kFbpTaps - 1; t += blockDim.x) {
-    int m = t - (half - 1);
-    if (m < 0) m += L;
-    // x[m] of the padded, extended row
-    int src;  // index into the padded row [0, np)
-    if (m < np) src = m;
-    else if (m < end) src = 2 * np - 1 - m;
-    else src = -1;
-    float v = 0.f;
-    if (src >= 0) v = r[min(max(src - 1, 0), nx - 1)];
-    e[t] = v;
+  int m = t - (kFbpTaps / 2 - 1);
+  if (m < 0) m += L;
+  // index into the padded row [0, np)
+  const int src = m < np ? m : m < end ? 2 * np - 1 - m : -1;
+  return src >= 0 ? r[min(max(src - 1, 0), nx - 1)] : 0.f;
+}
+
+__global__ void __launch_bounds__(256) fbp_filter_kernel(float *rows, int nx, int L, const FbpTaps taps) {
+  extern __shared__ double fsm[];
+  double *f = fsm;                 // [251]
+  double *e = fsm + kFbpTaps + 1;  // [fbp_slot(nx + 250 + kFbpRun)]
+  for (int k = threadIdx.x; k < kFbpTaps; k += blockDim.x) f[k] = (double)taps.f[k];
+  float *r = rows + (size_t)blockIdx.x * nx;
+  for (int t = threadIdx.x; t < nx + kFbpTaps - 1 + kFbpRun; t += blockDim.x)
+    e[fbp_slot(t)] = t < nx + kFbpTaps - 1 ? (double)fbp_sample(r, t, nx, L) : 0.0;
+  __syncthreads();
+  float *out = reinterpret_cast<float *>(e + fbp_slot(nx + kFbpTaps + 2 * kFbpRun));
+  for (int b0 = 0; b0 < nx; b0 += blockDim.x * kFbpRun) {
+    const int i0 = min(b0 + (int)threadIdx.x * kFbpRun, nx);
+    // out[i0 + m] = sum_k f[k] e[i0 + m + 250 - k]; the taps run from the last,
+    // so that the window moves up: step s has tap 250 - s and w[m] = e[i0 + s + m].
+    double acc[kFbpRun], w[kFbpRun];
+    const double *p = e + fbp_slot(i0);
+#pragma unroll
+    for (int m = 0; m < kFbpRun; ++m) acc[m] = 0.0, w[m] = p[m];
+    p += kFbpRun + 1;
+    // whole turns of the window: sample i0 + s + m sits in w[(s + m) % kFbpRun]
+    int s = 0;
+#pragma unroll 1
+    for (; s + kFbpRun <= kFbpTaps; s += kFbpRun, p += kFbpRun + 1) {
+#pragma unroll
+      for (int u = 0; u < kFbpRun; ++u) {
+        const double c = f[kFbpTaps - 1 - s - u];
+#pragma unroll
+        for (int m = 0; m < kFbpRun; ++m) acc[m] = fma(c, w[(u + m) % kFbpRun], acc[m]);
+        w[u] = p[u];  // sample i0 + s + u + kFbpRun takes the place of i0 + s + u
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kFbpTaps % kFbpRun; ++u) {
+      const double c = f[kFbpTaps % kFbpRun - 1 - u];
+#pragma unroll
+      for (int m = 0; m < kFbpRun; ++m) acc[m] = fma(c, w[(u + m) % kFbpRun], acc[m]);
+      w[u] = p[u];
+    }
+    // Through shared memory to the row (whose reads e holds a copy of), so that a
+    // warp writes consecutive samples.
+#pragma unroll
+    for (int m = 0; m < kFbpRun; ++m) out[threadIdx.x * (kFbpRun + 1) + m] = (float)acc[m];
+    __syncthreads();
+    for (int i = threadIdx.x; i < min((int)blockDim.x * kFbpRun, nx - b0); i += blockDim.x)
+      r[b0 + i] = out[i + i / kFbpRun];
+    __syncthreads();
   }
+}
+
+// Rows too long for shared memory in double (above about 25000 samples): the
+// samples in float, one output per thread.
+__global__ void __launch_bounds__(256)
+    fbp_filter_wide_kernel(float *rows, int nx, int L, const FbpTaps taps) {
+  extern __shared__ double fsm[];
+  double *f = fsm;                                       // [251]
+  float *e = reinterpret_cast<float *>(fsm + kFbpTaps);  // [nx + 250]
+  for (int k = threadIdx.x; k < kFbpTaps; k += blockDim.x) f[k] = (double)taps.f[k];
+  float *r = rows + (size_t)blockIdx.x * nx;
+  for (int t = threadIdx.x; t < nx + kFbpTaps - 1; t += blockDim.x) e[t] = fbp_sample(r, t, nx, L);
   __syncthreads();
   for (int i = threadIdx.x; i < nx; i += blockDim.x) {
     double acc = 0.0;
@@ -343,13 +405,24 @@ __global__ void __launch_bounds__(256) fbp_filter_kernel(float *rows, int nx, in
 
 cudaError_t launch_fbp_filter(float *rows, long long nrows, int nx, int L, int mode,
                               cudaStream_t s) {
-  const size_t smem = kFbpTaps * sizeof(double) + (size_t)(nx + kFbpTaps) * sizeof(float);
-  cudaError_t e = cudaFuncSetAttribute(fbp_filter_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const int threads = std::max(32, std::min(256, ((nx + kFbpRun - 1) / kFbpRun + 31) & ~31));
+  const size_t smem =
+      (kFbpTaps + 1 + (size_t)fbp_slot(nx + kFbpTaps + 2 * kFbpRun)) * sizeof(double) +
+      threads * (kFbpRun + 1) * sizeof(float);
+  const bool wide = smem > 220 * 1024;
+  const size_t wide_smem = kFbpTaps * sizeof(double) + (size_t)(nx + kFbpTaps) * sizeof(float);
+  cudaError_t e = cudaFuncSetAttribute(wide ? fbp_filter_wide_kernel : fbp_filter_kernel,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(wide ? wide_smem : smem));
   if (e != cudaSuccess) return e;
+  FbpTaps taps;
+  for (int k = 0; k < kFbpTaps; ++k) taps.f[k] = fbp_tap(k, mode);
   for (long long r0 = 0; r0 < nrows; r0 += 2147483647ll) {
     const unsigned n = (unsigned)std::min<long long>(nrows - r0, 2147483647ll);
-    fbp_filter_kernel<<<n, 256, smem, s>>>(rows + (size_t)r0 * nx, nx, L, mode);
+    if (wide)
+      fbp_filter_wide_kernel<<<n, 256, wide_smem, s>>>(rows + (size_t)r0 * nx, nx, L, taps);
+    else
+      fbp_filter_kernel<<<n, threads, smem, s>>>(rows + (size_t)r0 * nx, nx, L, taps);
   }
   return cudaGetLastError();
 }
@@ -361,53 +434,93 @@ cudaError_t launch_fbp_filter(float *rows, long long nrows, int nx, int L, int m
 // (nx/bin) x (ny/bin) with OpenCV's area resize: output pixel (i, j) is the
 // mean of the input over [i sx, (i+1) sx) x [j sy, (j+1) sy), sx = nx/(nx/bin),
 // partial pixels weighted by their overlap (an exact block mean when bin
-// divides the size).  One thread per output pixel, separable sums in FP64.
+// divides the size).
+//
+// Bound by HBM.  A CTA takes a run of pixels of one output row: its threads
+// read the cell's input rows along x, coalesced and all rows in flight, and
+// leave each column's weighted sum (FP64) in shared memory, from which each
+// output pixel adds its columns.  10 images of 4096 x 4096, bin 4: 318 -> 166 us
+// (one thread per output pixel, weights in local memory, before).
 
-__device__ __forceinline__ int area_axis(int n, int dn, int d, int *first, double *w, int cap) {
-  const double scale = (double)n / dn;
-  const double a = d * scale, b = a + scale > n ? (double)n : a + scale;
-  const int i0 = (int)floor(a), i1 = (int)ceil(b);
-  const double width = b - a;
-  int k = 0;
-  for (int i = i0; i < i1 && k < cap; ++i, ++k) {
-    const double lo = i > a ? i : a, hi = i + 1 < b ? i + 1 : b;
-    w[k] = (hi - lo) / width;
-  }
-  *first = i0;
-  return k;
+// Input cell [*first, *first + count) of output index d on an axis of n pixels
+// and scale pixels per output; lo and hi bound it, the overlap of pixel i is
+// min(i + 1, hi) - max(i, lo).
+__device__ __forceinline__ int area_cell(int n, double scale, int d, int *first, double *lo,
+                                         double *hi) {
+  *lo = d * scale;
+  *hi = *lo + scale > n ? (double)n : *lo + scale;
+  *first = (int)floor(*lo);
+  return (int)ceil(*hi) - *first;
+}
+__device__ __forceinline__ double area_overlap(int i, double lo, double hi) {
+  return (i + 1 < hi ? (double)(i + 1) : hi) - (i > lo ? (double)i : lo);
 }
 
-constexpr int kBinMax = 64;  // largest bin factor (weights per axis: bin + 1)
+constexpr int kBinMax = 64;  // largest bin factor; cells are less than two bins wide
+constexpr int kBinCols = 1024;  // input columns of a CTA (a single cell's may be fewer)
 
-__global__ void resample_bin_kernel(const float *__restrict__ src, int nx, int ny, int nt,
-                                    int dnx, int dny, float *__restrict__ dst) {
-  const size_t total = (size_t)dnx * dny * nt;
-  for (size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x; o < total;
-       o += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(o % dnx);
-    const size_t jt = o / dnx;
-    const int j = (int)(jt % dny), t = (int)(jt / dny);
-    double wx[kBinMax + 2], wy[kBinMax + 2];
-    int x0, y0;
-    const int kx = area_axis(nx, dnx, i, &x0, wx, kBinMax + 2);
-    const int ky = area_axis(ny, dny, j, &y0, wy, kBinMax + 2);
-    double acc = 0.0;
-    for (int b = 0; b < ky; ++b) {
-      const float *row = src + ((size_t)t * ny + y0 + b) * nx + x0;
-      double r = 0.0;
-      for (int a = 0; a < kx; ++a) r += wx[a] * (double)row[a];
-      acc += wy[b] * r;
+__global__ void __launch_bounds__(256)
+    resample_bin_kernel(const float *__restrict__ src, int nx, int ny, int dnx, int dny, double sx,
+                        double sy, double inv, int run, int j0, float *__restrict__ dst) {
+  __shared__ double col[kBinCols + 8];
+  __shared__ double wy[2 * kBinMax + 2];
+  const int j = j0 + blockIdx.y, t = blockIdx.z, i0 = blockIdx.x * run, i1 = min(dnx, i0 + run);
+  int y0, x0, last;
+  double lo, hi;
+  const int ky = area_cell(ny, sy, j, &y0, &lo, &hi);
+  if (threadIdx.x < ky) wy[threadIdx.x] = area_overlap(y0 + threadIdx.x, lo, hi) * inv;
+  area_cell(nx, sx, i0, &x0, &lo, &hi);
+  const int klast = area_cell(nx, sx, i1 - 1, &last, &lo, &hi), xe = last + klast;
+  __syncthreads();
+  const float *row0 = src + ((size_t)t * ny + y0) * nx;
+  // four columns per thread where the rows allow 16-byte reads
+  const bool vec = (nx & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
+  const int xs = vec ? x0 & ~3 : x0;
+  if (vec) {
+    for (int x = xs + 4 * threadIdx.x; x < xe; x += 1024) {
+      double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 8
+      for (int b = 0; b < ky; ++b) {
+        const float4 v = __ldg(reinterpret_cast<const float4 *>(row0 + (size_t)b * nx + x));
+        const double w = wy[b];
+        s[0] = fma(w, (double)v.x, s[0]);
+        s[1] = fma(w, (double)v.y, s[1]);
+        s[2] = fma(w, (double)v.z, s[2]);
+        s[3] = fma(w, (double)v.w, s[3]);
+      }
+#pragma unroll
+      for (int m = 0; m < 4; ++m) col[x - xs + m] = s[m];
     }
-    dst[o] = (float)acc;
+  } else {
+    for (int x = xs + threadIdx.x; x < xe; x += 256) {
+      double s = 0.0;
+#pragma unroll 8
+      for (int b = 0; b < ky; ++b) s = fma(wy[b], (double)__ldg(row0 + (size_t)b * nx + x), s);
+      col[x - xs] = s;
+    }
+  }
+  __syncthreads();
+  for (int i = i0 + threadIdx.x; i < i1; i += 256) {
+    int f;
+    const int k = area_cell(nx, sx, i, &f, &lo, &hi);
+    double acc = 0.0;
+    for (int a = f; a < f + k; ++a) acc = fma(area_overlap(a, lo, hi), col[a - xs], acc);
+    dst[((size_t)t * dny + j) * dnx + i] = (float)acc;
   }
 }
 
 cudaError_t launch_resample_bin(const float *src, int nx, int ny, int nt, int bin, float *dst,
                                 cudaStream_t s) {
   const int dnx = nx / bin, dny = ny / bin;
-  const size_t total = (size_t)dnx * dny * nt;
-  const unsigned blocks = (unsigned)std::min<size_t>((total + 255) / 256, 148 * 16);
-  resample_bin_kernel<<<blocks > 0 ? blocks : 1, 256, 0, s>>>(src, nx, ny, nt, dnx, dny, dst);
+  const double sx = (double)nx / dnx, sy = (double)ny / dny;
+  // The run's cells span at most kBinCols columns and a part of one at each end.
+  const int run = std::max(1, std::min(dnx, (int)(kBinCols * (double)dnx / nx)));
+  const unsigned gx = (unsigned)((dnx + run - 1) / run);
+  for (int t0 = 0; t0 < nt; t0 += 65535)
+    for (int j0 = 0; j0 < dny; j0 += 65535)
+      resample_bin_kernel<<<dim3(gx, std::min(65535, dny - j0), std::min(65535, nt - t0)), 256, 0,
+                            s>>>(src + (size_t)t0 * nx * ny, nx, ny, dnx, dny, sx, sy,
+                                 1.0 / (sx * sy), run, j0, dst + (size_t)t0 * dnx * dny);
   return cudaGetLastError();
 }
 
