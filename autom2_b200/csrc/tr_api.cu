@@ -71,6 +71,7 @@ struct tr_ctx {
   double *admm_dot_d = nullptr;   // ADMM: dot partials + the 3 CG scalars
   bool wt_ready = false, wtvol_ready = false;
   int filt_nx = 0, filt_npad = 0, filt_log2m = 0;
+  size_t filt_ramp = 0;  // the short form's vectors behind the twiddles, 0: none
   float2 *ghat_d = nullptr, *tw_d = nullptr;
   float *hproj_d = nullptr, *hvol_d = nullptr;
   // byte output: slab partial sums and statistics, the bytes themselves
@@ -395,7 +396,7 @@ tr_status build_filter(tr_ctx *c, int nx) {
     return TR_OK;
   }
   RweightSpectrum sp;
-  if (!rweight_spectrum(nx, kSmemMax, &sp))
+  if (!rweight_plan(nx, kSmemMax, &sp))
     return fail(c, TR_ERR_UNSUPPORTED, "row length %d needs an FFT of %d points", nx,
                 1 << sp.log2m);
   const int M = 1 << sp.log2m;
@@ -403,11 +404,15 @@ tr_status build_filter(tr_ctx *c, int nx) {
   scratch_free(c, (void **)&c->tw_d);
   tr_status s = scratch_alloc(c, (void **)&c->ghat_d, sizeof(float2) * M, "filter spectrum");
   if (s) return s;
-  s = scratch_alloc(c, (void **)&c->tw_d, sizeof(float2) * sp.tw.size(), "filter twiddles");
+  const size_t ntw = sp.tw.size();
+  s = scratch_alloc(c, (void **)&c->tw_d, sizeof(float2) * (ntw + sp.ramp.size()),
+                    "filter twiddles");
   if (s) return s;
   TR_CUDA(c, cudaMemcpy(c->ghat_d, sp.ghat.data(), sizeof(float2) * M, cudaMemcpyHostToDevice));
+  sp.tw.insert(sp.tw.end(), sp.ramp.begin(), sp.ramp.end());
   TR_CUDA(c, cudaMemcpy(c->tw_d, sp.tw.data(), sizeof(float2) * sp.tw.size(),
                         cudaMemcpyHostToDevice));
+  c->filt_ramp = sp.ramp.empty() ? 0 : ntw;
   c->filt_nx = nx;
   c->filt_npad = sp.npad;
   c->filt_log2m = sp.log2m;
@@ -903,6 +908,7 @@ tr_status tr_filter_rweight(tr_ctx *c, float *proj, void *stream) {
   f.log2m = c->filt_log2m;
   f.ghat = c->ghat_d;
   f.tw = c->tw_d;
+  f.ramp = c->filt_ramp ? c->tw_d + c->filt_ramp : nullptr;
   TR_CUDA(c, launch_rweight(f, (cudaStream_t)stream));
   return TR_OK;
 }

@@ -39,7 +39,7 @@ constexpr int kRweightMinLog2 = 4;
 constexpr int kRweightMaxLog2 = 14;
 
 struct RweightSpectrum {
-  int npad = 0;   // padded row length nx + nx/10 of the reference
+  int npad = 0;   // row length of the transform: nx + nx/10 as the reference pads it, or nx
   int log2m = 0;  // FFT size 2^log2m >= npad + nx - 1
   std::vector<float2> ghat;  // kernel spectrum, natural order, scaled 1/(M nx)
   // Twiddles of the radix-16 Stockham passes with sub-transform size
@@ -47,18 +47,14 @@ struct RweightSpectrum {
   // table per pass in that order: entry [r - 1][k] = e^{-2 pi i r k / (16 Ns)}
   // for r = 1..15, k < Ns.
   std::vector<float2> tw;
+  // Short form (rweight_plan): output j gains ramp[j].x times the row's first
+  // sample and ramp[j].y times its last; empty in the padded form.
+  std::vector<float2> ramp;
 };
 
-// False when the FFT (M points plus one pad entry per 16) would not fit
-// `smem_max` bytes of shared memory.
-inline bool rweight_spectrum(int nx, size_t smem_max, RweightSpectrum *out) {
-  const int N = nx + nx / 10;
-  int log2m = kRweightMinLog2;
-  while ((1 << log2m) < N + nx - 1) ++log2m;
-  const int M = 1 << log2m;
-  out->npad = N;
-  out->log2m = log2m;
-  if ((size_t)(M + M / 16) * sizeof(float2) > smem_max || log2m > kRweightMaxLog2) return false;
+// h[d], d in [0, N): the filter as a circular convolution of the padded row
+// (N = nx + nx/10 samples), unscaled.
+inline std::vector<double> rweight_kernel_taps(int N) {
   // Weights exactly as filter_prj.cpp:694-723 forms them (float arithmetic).
   const int r = (int)floor((float)N * 0.05f);
   const float sg = (float)N * 0.5f;
@@ -82,8 +78,15 @@ inline bool rweight_spectrum(int nx, size_t smem_max, RweightSpectrum *out) {
     if (N % 2 == 0) acc += (d % 2 == 0) ? W[N / 2] : -W[N / 2];
     h[d] = acc;
   }
+  return h;
+}
+
+// Spectrum of the lags lo..hi of h on M = 2^log2m points, and the twiddles.
+inline void rweight_tables(int nx, const std::vector<double> &h, int lo, int hi, int log2m,
+                           RweightSpectrum *out) {
+  const int M = 1 << log2m, N = (int)h.size();
   std::vector<std::complex<double>> g(M, 0.0);
-  for (int e = -(N - 1); e <= nx - 1; ++e) g[(e % M + M) % M] = h[(e % N + N) % N];
+  for (int e = lo; e <= hi; ++e) g[(e % M + M) % M] = h[(e % N + N) % N];
   fft_host(g);
   out->ghat.resize(M);
   const double scale = 1.0 / ((double)M * nx);
@@ -100,6 +103,58 @@ inline bool rweight_spectrum(int nx, size_t smem_max, RweightSpectrum *out) {
       }
   }
   if (out->tw.empty()) out->tw.push_back(make_float2(1.f, 0.f));  // keep the buffer non-empty
+  out->ramp.clear();
+}
+
+// False when the FFT (M points plus one pad entry per 16) would not fit
+// `smem_max` bytes of shared memory.
+inline bool rweight_spectrum(int nx, size_t smem_max, RweightSpectrum *out) {
+  const int N = nx + nx / 10;
+  int log2m = kRweightMinLog2;
+  while ((1 << log2m) < N + nx - 1) ++log2m;
+  const int M = 1 << log2m;
+  out->npad = N;
+  out->log2m = log2m;
+  if ((size_t)(M + M / 16) * sizeof(float2) > smem_max || log2m > kRweightMaxLog2) return false;
+  rweight_tables(nx, rweight_kernel_taps(N), -(N - 1), nx - 1, log2m, out);
+  return true;
+}
+
+// The form the device runs for rows of nx samples; refuses what
+// rweight_spectrum does.
+//
+// The row's pad is a ramp between its last sample and its first, so what it
+// adds to the outputs is two fixed vectors times those samples (`ramp`).
+// Without it the convolution spans the lags -(nx-1)..nx-1 only, 2 nx - 1 where
+// the padded row's spans 2.1 nx: for row lengths that are a power of two, and
+// up to 5 % below one, the transform is half as long.  Elsewhere the padded
+// form stands: the transforms are the same and it has no vectors to read.
+inline bool rweight_plan(int nx, size_t smem_max, RweightSpectrum *out) {
+  const int N = nx + nx / 10;
+  int log2m = kRweightMinLog2;
+  while ((1 << log2m) < 2 * nx - 1) ++log2m;
+  int padded = log2m;
+  while ((1 << padded) < N + nx - 1) ++padded;
+  if (padded == log2m) return rweight_spectrum(nx, smem_max, out);
+  const int P = 1 << padded;
+  out->npad = N;
+  out->log2m = padded;
+  if ((size_t)(P + P / 16) * sizeof(float2) > smem_max || padded > kRweightMaxLog2) return false;
+  out->npad = nx;
+  out->log2m = log2m;
+  const std::vector<double> h = rweight_kernel_taps(N);
+  rweight_tables(nx, h, -(nx - 1), nx - 1, log2m, out);
+  out->ramp.resize(nx);
+  const int nxp = N - nx + 1;
+  for (int j = 0; j < nx; ++j) {
+    double first = 0, last = 0;
+    for (int m = nx; m < N; ++m) {
+      const double k = h[((j - m) % N + N) % N];
+      first += k * (double)((float)(m - nx + 1) / (float)nxp);
+      last += k * (double)((float)(N - m) / (float)nxp);
+    }
+    out->ramp[j] = make_float2((float)(first / nx), (float)(last / nx));
+  }
   return true;
 }
 

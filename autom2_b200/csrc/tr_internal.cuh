@@ -166,6 +166,7 @@ struct FilterArgs {
   int log2m;            // M = 1 << log2m
   const float2 *ghat;   // [M] kernel spectrum, natural order, scaled
   const float2 *tw;     // two-level twiddles (tr_filter_host.h RweightSpectrum::tw)
+  const float2 *ramp;   // [nx] of the short form (RweightSpectrum::ramp), else nullptr
 };
 
 // ------------------------------------------------------------ batched steps

@@ -242,15 +242,16 @@ tr_status ensure_filter(tr_sched *S, int nx, std::pair<float2 *, float2 *> *out)
     return TR_OK;
   }
   RweightSpectrum sp;
-  if (!rweight_spectrum(nx, kSchedSmemMax, &sp))
+  if (!rweight_plan(nx, kSchedSmemMax, &sp))
     return sched_fail(S, TR_ERR_UNSUPPORTED, "row length too long for the filter");
   const int M = 1 << sp.log2m;
   float2 *g = nullptr, *t = nullptr;
   SCHED_CUDA(S, cudaMalloc(&g, sizeof(float2) * M));
-  SCHED_CUDA(S, cudaMalloc(&t, sizeof(float2) * sp.tw.size()));
+  std::vector<float2> tw = sp.tw;  // the ramp vectors behind the twiddles
+  tw.insert(tw.end(), sp.ramp.begin(), sp.ramp.end());
+  SCHED_CUDA(S, cudaMalloc(&t, sizeof(float2) * tw.size()));
   SCHED_CUDA(S, cudaMemcpy(g, sp.ghat.data(), sizeof(float2) * M, cudaMemcpyHostToDevice));
-  SCHED_CUDA(S, cudaMemcpy(t, sp.tw.data(), sizeof(float2) * sp.tw.size(),
-                           cudaMemcpyHostToDevice));
+  SCHED_CUDA(S, cudaMemcpy(t, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice));
   S->filt[nx] = {g, t};
   S->filt_h[nx] = sp;
   *out = {g, t};
@@ -330,6 +331,7 @@ tr_status admit(tr_sched *S, Job &j) {
     f.log2m = sp.log2m;
     f.ghat = filt.first;
     f.tw = filt.second;
+    f.ramp = sp.ramp.empty() ? nullptr : filt.second + sp.tw.size();
     SCHED_CUDA(S, launch_rweight(f, ps));
   }
   if (!j.d.vol_in)

@@ -105,3 +105,24 @@ def test_two_streams_share_a_context(engine, restatement):
     want = R.backproject(R.geom(nx, ny, nt, th, layout, 0, org), c8, proj, 0 * vol, fp64=True)
     for b, s in zip(v, (1.0, -3.0)):
         assert O.rel_l2(b.cpu().numpy(), s * want) < TOL
+
+
+def test_an_infinite_edge_pixel_stays_inside_the_image(engine, restatement):
+    """Voxels that no pixel reaches get nothing, also beside a pixel that is not
+    finite, and voxels between it and its neighbour are not finite."""
+    R = restatement
+    nx, ny, nt, th = 256, 128, 3, 64
+    c8 = R.coeffs(np.array([-40, 0.5, 30], np.float32), 0.0, 0.0, 0.0)
+    proj = np.random.default_rng(3).normal(size=(nt, ny, nx)).astype(np.float32)
+    proj[0, 5, 0] = np.inf
+    proj[2, 9, nx - 1] = -np.inf
+    org = T.default_origin(0, nx, ny, th)
+    engine.set_problem(nx, ny, nt, th, c8, T.LAYOUT_Y, org)
+    v = torch.zeros((ny, th, nx), device="cuda")
+    engine.backproject(torch.from_numpy(proj).cuda(), v)
+    want = R.backproject(R.geom(nx, ny, nt, th, 0, 0, org), c8, proj, np.zeros((ny, th, nx)),
+                         fp64=True)
+    got = v.cpu().numpy()
+    np.testing.assert_array_equal(np.isfinite(got), np.isfinite(want))
+    ok = np.isfinite(want)
+    assert O.rel_l2(got[ok], want[ok]) < TOL
