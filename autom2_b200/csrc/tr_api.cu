@@ -43,7 +43,8 @@ struct tr_ctx {
   int fw = 0, fh = 0, chunk_bp = 1, chunk_fp = 1;
   int ffw = 0, ffh = 0;  // forward-projection tile window
   float fp_nbound = 0;   // most voxel contributions per forward window entry
-  TiltGeo *geo_d = nullptr;
+  TiltGeo *geo_d = nullptr;  // kept across problems, grown to the most tilts seen
+  int geo_cap = 0;
 
   // scratch: buffers are kept across problems and grown on demand; slot
   // records each buffer's capacity and the problem generation that last
@@ -209,10 +210,6 @@ bool scratch_try(tr_ctx *c, void **p, size_t bytes) {
 // problem to reuse (a new generation: they count as idle until claimed).
 void release_problem(tr_ctx *c) {
   ++c->gen;
-  if (c->geo_d) {
-    cudaFree(c->geo_d);
-    c->geo_d = nullptr;
-  }
   c->wt_ready = c->wtvol_ready = false;
   c->have_problem = false;
 }
@@ -848,6 +845,7 @@ tr_status tr_destroy(tr_ctx *c) {
   if (c->ev_start) cudaEventDestroy(c->ev_start);
   if (c->ev_rows) cudaEventDestroy(c->ev_rows);
   if (c->err_d) cudaFree(c->err_d);
+  if (c->geo_d) cudaFree(c->geo_d);
   delete c;
   return TR_OK;
 }
@@ -871,13 +869,14 @@ tr_status tr_set_problem(tr_ctx *c, int nx, int ny, int nt, int th, int layout,
   c->ny = ny;
   c->nt = nt;
   c->th = th;
-  TR_CUDA(c, cudaMalloc(&c->geo_d, sizeof(TiltGeo) * nt));
-  tr_status st = load_geometry(c, coeff8, nullptr);
-  if (st) {
+  if (nt > c->geo_cap) {
     cudaFree(c->geo_d);
     c->geo_d = nullptr;
-    return st;
+    c->geo_cap = 0;
+    TR_CUDA(c, cudaMalloc(&c->geo_d, sizeof(TiltGeo) * nt));
+    c->geo_cap = nt;
   }
+  TR_TRY(load_geometry(c, coeff8, nullptr));
   c->layout = layout;
   c->ox = ox;
   c->oy = oy;
