@@ -293,7 +293,7 @@ bool rows_path(const tr_ctx *c, const RowsRule &r, int nz, int nt, cudaStream_t 
   }
   return cs == cudaStreamCaptureStatusNone;
 }
-static_assert(kRowBpX == kRowFpX && kRowBpZ == kRowFpZ && kTZ == kFTZ, "one tile for the rule");
+static_assert(kTZ == kFTZ, "one section tile for the rule");
 // Orders `s` after the row buffers' last use, on whichever stream that was, and
 // marks their use so far on `s` as the last.
 cudaError_t rows_acquire(tr_ctx *c, cudaStream_t s) {

@@ -66,7 +66,7 @@ inline float fp_entry_bound_sep(double min_a1) {
 // Voxels along x and z of a row-invariant tile (tr_rows.cu): back-projection
 // and forward projection.
 constexpr int kRowBpX = 16, kRowBpZ = 8;
-constexpr int kRowFpX = 16, kRowFpZ = 8;
+constexpr int kRowFpX = 16, kRowFpZ = 4;
 
 // Fills g[0..nt) and *out from [nt][8] coefficients; *bad_tilt names the
 // offending tilt for the per-tilt failures.

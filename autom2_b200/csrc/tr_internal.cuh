@@ -31,9 +31,9 @@ constexpr int kFTZ = kZG * kFNV;              // 32
 constexpr int kMaxWindow = 511;
 
 // Row-invariant geometries (tr_rows.cu): rows of a tile, and the shared memory
-// a CTA may take, alone on its SM or as one of two.
+// an SM's tiles may take together (1 KB a tile is the system's).
 constexpr int kRowTile = 128;
-constexpr size_t kRowSmem = 220 * 1024, kRowSmem2 = 113 * 1024;
+constexpr size_t kRowSmem = 224 * 1024;
 
 // Per-tilt projection geometry.  a/b are the reference's linear coefficients
 // (detector x = a0 + a1 X + a2 Y + a3 Z + ox, y likewise with b, X/Y/Z the

@@ -224,9 +224,11 @@ __device__ __forceinline__ void load_quad(const float *p, bool in, bool vec, int
   }
 }
 
-constexpr int kBpWarps = 8;
+// Patches of a tile along x and z, a warp each; tiles per SM at 16 warps.
+constexpr int kBpPX = kRowBpX / 4, kBpPZ = kRowBpZ / 4, kBpWarps = kBpPX * kBpPZ;
+constexpr int kBpPerSm = 16 / kBpWarps;
+constexpr int kBpQuads = 4 * kBpPZ * kBpPX;  // float4s of a tile's row, all sections
 constexpr int kLag = 4;  // a stage is refilled kLag tilts after its use
-constexpr int kBpX = kRowBpX, kBpZ = kRowBpZ;  // voxels of a tile along x and z
 
 // Back-projection.  Volume tile of 16 (x) x 8 (z) voxels and 128 rows; warp w
 // owns the patch at ((w % 4) 4, (w / 4) 4).  Tilts come through a ring of stages; the warps
@@ -240,11 +242,11 @@ constexpr int kBpX = kRowBpX, kBpZ = kRowBpZ;  // voxels of a tile along x and z
 // 1024 x 1024 x 256 voxels, 61 tilts: 3.83 ms with the row stack's 0.15 ms,
 // from 6.69 ms by the general kernel (4.3e12 from 2.4e12 voxel-tilts/s).
 template <int MODE>
-__global__ void __launch_bounds__(kBpWarps * 32, 2)
+__global__ void __launch_bounds__(kBpWarps * 32, kBpPerSm)
     bp_rows_kernel(const BpArgs a, const float *__restrict__ rows, int cols, int stages) {
   extern __shared__ __align__(128) unsigned char dsm[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int xc = blockIdx.x * kBpX, zl = blockIdx.y * kBpZ, yc = blockIdx.z * kRowTile;
+  const int xc = blockIdx.x * kRowBpX, zl = blockIdx.y * kRowBpZ, yc = blockIdx.z * kRowTile;
   const int nt = a.nt;
   const unsigned win_bytes = (unsigned)cols * kColBytes;
   const unsigned stage_bytes = win_bytes + kBpWarps * (unsigned)sizeof(PatchPath);
@@ -259,7 +261,7 @@ __global__ void __launch_bounds__(kBpWarps * 32, 2)
     }
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   for (int i = tid; i < nt; i += blockDim.x)
-    tt[i] = row_tilt(a.geo[a.t0 + i], xc, zl + a.v.zoff, a.ox, a.oz, kBpX - 1, kBpZ - 1, a.img.nx,
+    tt[i] = row_tilt(a.geo[a.t0 + i], xc, zl + a.v.zoff, a.ox, a.oz, kRowBpX - 1, kRowBpZ - 1, a.img.nx,
                      cols);
   __syncthreads();
 
@@ -275,7 +277,7 @@ __global__ void __launch_bounds__(kBpWarps * 32, 2)
 #pragma unroll 1
     for (int b = 0; b < kBpWarps / 2; ++b) {
       const int w = 2 * b + (lane >> 4);
-      path_records<false>(tl, (w & 3) * 4, (w >> 2) * 4, lane, a.img.nx, paths + w);
+      path_records<false>(tl, w % kBpPX * 4, w / kBpPX * 4, lane, a.img.nx, paths + w);
     }
     __syncwarp();
     if (lane == 0) mbar_expect_tx(full + s, win_bytes);  // the stage's one arrival
@@ -284,8 +286,8 @@ __global__ void __launch_bounds__(kBpWarps * 32, 2)
 
   // The tile's voxels are read at the end: into L2 meanwhile, one 64-byte
   // segment (a section's 16 x) per row and section.
-  for (int i = tid; i < kRowTile * kBpZ; i += kBpWarps * 32) {
-    const int y = yc + i / kBpZ, z = zl + i % kBpZ;
+  for (int i = tid; i < kRowTile * kRowBpZ; i += kBpWarps * 32) {
+    const int y = yc + i / kRowBpZ, z = zl + i % kRowBpZ;
     if (y < a.v.ny && z < a.v.nz)
       asm volatile("prefetch.global.L2 [%0];" ::"l"(a.v.vol + (size_t)y * a.v.sy +
                                                      (size_t)z * a.v.sz + xc));
@@ -343,9 +345,9 @@ __global__ void __launch_bounds__(kBpWarps * 32, 2)
   // Epilogue.  The sums go through shared memory, [row][section][16 x] with
   // the 16-byte pieces of a row exchanged so that neither side meets in a
   // bank, and the volume is read and written by sections' rows of 64 bytes.
-  float4 *sum = reinterpret_cast<float4 *>(dsm);  // [128][32]
+  float4 *sum = reinterpret_cast<float4 *>(dsm);  // [128][kBpQuads]
   {
-    const int px = warp & 3, pz = (warp >> 2) * 4;
+    const int px = warp % kBpPX, pz = warp / kBpPX * 4;
 #pragma unroll
     for (int r = 0; r < kLaneRows; ++r)
 #pragma unroll
@@ -357,23 +359,26 @@ __global__ void __launch_bounds__(kBpWarps * 32, 2)
           unpack2(acc[k * 4 + x][r >> 1], lo, hi);
           f[x] = r & 1 ? hi : lo;
         }
-        sum[(lane * 4 + r) * 32 + (((pz + k) * 4 + px) ^ (lane & 7))] =
+        sum[(lane * 4 + r) * kBpQuads + (((pz + k) * kBpPX + px) ^ (lane & 7))] =
             make_float4(f[0], f[1], f[2], f[3]);
       }
   }
   __syncthreads();
-  const int x0 = xc + (lane & 3) * 4, z = zl + (lane >> 2);
+  const int quad = lane % kBpQuads;
+  const int x0 = xc + quad % kBpPX * 4, z = zl + quad / kBpPX;
   const bool inz = z < a.v.nz && x0 < a.v.nx;
   const bool vec = rows_vec(a.v, x0);
   const int gx = (a.v.nx + kTX - 1) / kTX, gy = (a.v.ny + kTY - 1) / kTY;
   constexpr int kBatch = 8;  // rows whose reads are in flight together
+  constexpr int kStep = 32 / kBpQuads;  // rows a warp takes at a time
+  const int row0 = warp * (kRowTile / kBpWarps) + lane / kBpQuads;
 #pragma unroll 1
-  for (int i0 = 0; i0 < kRowTile / kBpWarps; i0 += kBatch) {
+  for (int i0 = 0; i0 < kRowTile / kBpWarps / kStep; i0 += kBatch) {
     float old[kBatch][4], scale[kBatch];
     int slot[kBatch];
 #pragma unroll
     for (int i = 0; i < kBatch; ++i) {
-      const int y = yc + warp * (kRowTile / kBpWarps) + i0 + i;
+      const int y = yc + row0 + (i0 + i) * kStep;
       const bool in = inz && y < a.v.ny;
       load_quad(a.v.vol + (size_t)y * a.v.sy + (size_t)z * a.v.sz + x0, in, vec, a.v.nx - x0,
                 old[i]);
@@ -386,9 +391,9 @@ __global__ void __launch_bounds__(kBpWarps * 32, 2)
     }
 #pragma unroll
     for (int i = 0; i < kBatch; ++i) {
-      const int row = warp * (kRowTile / kBpWarps) + i0 + i, y = yc + row;
+      const int row = row0 + (i0 + i) * kStep, y = yc + row;
       if (!inz || y >= a.v.ny) continue;
-      const float4 q = sum[row * 32 + (lane ^ ((row >> 2) & 7))];
+      const float4 q = sum[row * kBpQuads + (quad ^ ((row >> 2) & 7))];
       const float s[4] = {q.x, q.y, q.z, q.w};
       const float sc = MODE == BP_SIRT ? (scale[i] != 0.f ? a.gamma / scale[i] : 0.f) : a.gamma;
 #pragma unroll
@@ -479,10 +484,11 @@ __device__ __forceinline__ void splat_patch(const f32x2 (&vox)[16][2], unsigned 
   add_col(win + m.w, od0, od1);
 }
 
-constexpr int kFpWarps = 8;
-constexpr int kFpX = kRowFpX, kFpZ = kRowFpZ;
+constexpr int kFpPX = kRowFpX / 4, kFpPZ = kRowFpZ / 4, kFpWarps = kFpPX * kFpPZ;
+constexpr int kFpPerSm = 16 / kFpWarps;
+constexpr int kFpQuads = 4 * kFpPZ * kFpPX;
 
-// Forward projection of a tile of 16 (x) x 8 (z) voxels and 128 rows into the
+// Forward projection of a tile of 16 (x) x 4 (z) voxels and 128 rows into the
 // row stack.  The voxels stay in registers.  The tilts' windows stand in a
 // ring of slots and go from warp to warp: warp w adds its patch to a tilt's
 // window once warp w - 1 has, so that no two add to it at a time and the
@@ -493,48 +499,51 @@ constexpr int kFpX = kRowFpX, kFpZ = kRowFpZ;
 //
 // Bound as the back-projection, with more instructions (7 per voxel and tilt):
 // a column that leaves the path is a read, an addition and a write of its
-// window.  1024 x 1024 x 256 voxels, 61 tilts: 6.07 ms with the row sums'
+// window.  1024 x 1024 x 256 voxels, 61 tilts: 5.74 ms with the row sums'
 // conversion, from 8.12 ms by the general splat, whose 32-bit fixed point this
-// replaces by float sums.
-__global__ void __launch_bounds__(kFpWarps * 32, 2)
+// replaces by float sums.  Four warps in the chain and four CTAs per SM: eight
+// and two took 6.07 ms, an 8 x 8 tile 5.90 ms, two warps 5.87 ms.
+__global__ void __launch_bounds__(kFpWarps * 32, kFpPerSm)
     fp_rows_kernel(const FpArgs a, float *__restrict__ rows, int cols, int slots, int ahead) {
   extern __shared__ __align__(128) unsigned char dsm[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int xc = blockIdx.x * kFpX, zl = blockIdx.y * kFpZ, yc = blockIdx.z * kRowTile;
+  const int xc = blockIdx.x * kRowFpX, zl = blockIdx.y * kRowFpZ, yc = blockIdx.z * kRowTile;
   const int nt = a.nt;
   const unsigned win_bytes = (unsigned)cols * kColBytes;
   // the windows' room also holds the tile's voxels at first
-  RowTilt *tt = reinterpret_cast<RowTilt *>(dsm + max(slots * win_bytes, (unsigned)kRowTile * 512));
+  RowTilt *tt = reinterpret_cast<RowTilt *>(dsm + max(slots * win_bytes, (unsigned)kRowTile * kFpQuads * 16));
   PatchPath *paths = reinterpret_cast<PatchPath *>(tt + ((nt + 1) & ~1)) + warp * 2;
-  // per slot: warp w < 7 has added to it; [7]: it may be used again
+  // per slot: warp w has added to it; the last: it may be used again
   unsigned long long *hand = reinterpret_cast<unsigned long long *>(
       reinterpret_cast<PatchPath *>(tt + ((nt + 1) & ~1)) + kFpWarps * 2);
   for (int i = tid; i < slots * kFpWarps; i += blockDim.x) mbar_init(hand + i, 1);
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   for (int i = tid; i < nt; i += blockDim.x)
-    tt[i] = row_tilt(a.geo[a.t0 + i], xc, zl + a.v.zoff, a.ox, a.oz, kFpX - 1, kFpZ - 1, a.pnx, cols);
+    tt[i] = row_tilt(a.geo[a.t0 + i], xc, zl + a.v.zoff, a.ox, a.oz, kRowFpX - 1, kRowFpZ - 1, a.pnx, cols);
 
   // The tile's voxels, read by sections' rows of 64 bytes, through shared memory
   // (the windows') to the lanes that own their rows, as in the back-projection.
   f32x2 vox[16][2];
   bool any = a.v.vol == nullptr;
   if (a.v.vol) {
-    float4 *buf = reinterpret_cast<float4 *>(dsm);  // [128][32]
-    const int x0 = xc + (lane & 3) * 4, z = zl + (lane >> 2);
+    float4 *buf = reinterpret_cast<float4 *>(dsm);  // [128][kFpQuads]
+    const int quad = lane % kFpQuads;
+    const int x0 = xc + quad % kFpPX * 4, z = zl + quad / kFpPX;
     const bool inz = z < a.v.nz, vec = rows_vec(a.v, x0);
+    constexpr int kStep = 32 / kFpQuads;
 #pragma unroll 8
-    for (int i = 0; i < kRowTile / kFpWarps; ++i) {
-      const int row = warp * (kRowTile / kFpWarps) + i, y = yc + row;
+    for (int i = 0; i < kRowTile / kFpWarps / kStep; ++i) {
+      const int row = warp * (kRowTile / kFpWarps) + lane / kFpQuads + i * kStep, y = yc + row;
       float f[4];
       load_quad(a.v.vol + (size_t)y * a.v.sy + (size_t)z * a.v.sz + x0, inz && y < a.v.ny, vec,
                 a.v.nx - x0, f);
-      buf[row * 32 + (lane ^ ((row >> 2) & 7))] = make_float4(f[0], f[1], f[2], f[3]);
+      buf[row * kFpQuads + (quad ^ ((row >> 2) & 7))] = make_float4(f[0], f[1], f[2], f[3]);
       any |= f[0] != 0.f || f[1] != 0.f || f[2] != 0.f || f[3] != 0.f;
     }
   }
   if (!__syncthreads_or(any)) return;  // an all-zero tile adds nothing
   {
-    const int px = warp & 3, pz = (warp >> 2) * 4;
+    const int px = warp % kFpPX, pz = warp / kFpPX * 4;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       float4 f[4];
@@ -542,7 +551,7 @@ __global__ void __launch_bounds__(kFpWarps * 32, 2)
       for (int r = 0; r < 4; ++r) {
         if (a.v.vol) {
           f[r] = reinterpret_cast<const float4 *>(
-              dsm)[(lane * 4 + r) * 32 + (((pz + k) * 4 + px) ^ (lane & 7))];
+              dsm)[(lane * 4 + r) * kFpQuads + (((pz + k) * kFpPX + px) ^ (lane & 7))];
         } else {
           const int x0 = xc + px * 4;
           const bool in = yc + lane * 4 + r < a.v.ny && zl + pz + k < a.v.nz;
@@ -562,11 +571,11 @@ __global__ void __launch_bounds__(kFpWarps * 32, 2)
     // Into L2: the voxels of the tile that takes this one's place on the SM.
     unsigned n = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x + ahead;
     const unsigned bx = n % gridDim.x, by = n / gridDim.x % gridDim.y, bz = n / gridDim.x / gridDim.y;
-    for (int i = tid; i < kRowTile * kFpZ; i += blockDim.x) {
-      const int y = bz * kRowTile + i / kFpZ, z = by * kFpZ + i % kFpZ;
+    for (int i = tid; i < kRowTile * kRowFpZ; i += blockDim.x) {
+      const int y = bz * kRowTile + i / kRowFpZ, z = by * kRowFpZ + i % kRowFpZ;
       if (y < a.v.ny && z < a.v.nz)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(a.v.vol + (size_t)y * a.v.sy +
-                                                       (size_t)z * a.v.sz + bx * kFpX));
+                                                       (size_t)z * a.v.sz + bx * kRowFpX));
     }
   }
 
@@ -578,7 +587,7 @@ __global__ void __launch_bounds__(kFpWarps * 32, 2)
   for (int t = 0; t < nt; ++t) {
     if (!(t & 1)) {  // this warp's paths of two tilts
       __syncwarp();
-      path_records<true>(tt[min(t + (lane >> 4), nt - 1)], (warp & 3) * 4, (warp >> 2) * 4, lane,
+      path_records<true>(tt[min(t + (lane >> 4), nt - 1)], warp % kFpPX * 4, warp / kFpPX * 4, lane,
                          a.pnx, paths + (lane >> 4));
       __syncwarp();
     }
@@ -777,27 +786,27 @@ cudaError_t launch_unblend_rows(const float *rows, const TiltGeo *geo, int t0, i
 // Dynamic shared memory of the kernels.
 static size_t bp_rows_smem(int cols, int nt, int stages) {
   return (size_t)stages * (cols * kColBytes + kBpWarps * sizeof(PatchPath) + 16) +
-         (size_t)((nt + 1) & ~1) * sizeof(RowTilt);  // at least kRowTile * 512 for the epilogue
+         (size_t)((nt + 1) & ~1) * sizeof(RowTilt);  // at least the epilogue's sums
 }
 static int bp_rows_stages(int cols, int nt) {
   const size_t fixed = bp_rows_smem(cols, nt, 0), per = bp_rows_smem(cols, 0, 1);
-  if (fixed >= kRowSmem) return 0;
-  // two CTAs per SM when that leaves windows in flight
-  if (fixed < kRowSmem2 && (kRowSmem2 - fixed) / per >= kLag + 2)
-    return (int)std::min<size_t>(10, (kRowSmem2 - fixed) / per);
-  return (int)std::min<size_t>(10, (kRowSmem - fixed) / per);
+  // 16 warps per SM when that leaves windows in flight
+  for (size_t room : {kRowSmem / kBpPerSm, kRowSmem})
+    if (fixed < room && (room - fixed) / per >= kLag + 2)
+      return (int)std::min<size_t>(10, (room - fixed) / per);
+  return 0;
 }
 bool bp_rows_fits(int cols, int nt) { return bp_rows_stages(cols, nt) >= kLag + 2; }
 
 static size_t fp_rows_smem(int cols, int nt, int slots) {
-  return std::max<size_t>((size_t)slots * cols * kColBytes, kRowTile * 512) +
+  return std::max<size_t>((size_t)slots * cols * kColBytes, kRowTile * kFpQuads * 16) +
          (size_t)((nt + 1) & ~1) * sizeof(RowTilt) + kFpWarps * 2 * sizeof(PatchPath) +
          slots * kFpWarps * sizeof(unsigned long long);
 }
-// Slots: eight are in the warps' hands, one is being sent out.
+// Slots: one in each warp's hands, one being sent out, and some to spare.
 static int fp_rows_slots(int cols, int nt) {
-  for (size_t room : {kRowSmem2, kRowSmem})
-    for (int n = 11; n >= 9; --n)
+  for (size_t room : {kRowSmem / kFpPerSm, kRowSmem})
+    for (int n = kFpWarps + 4; n > kFpWarps; --n)
       if (fp_rows_smem(cols, nt, n) <= room) return n;
   return 0;
 }
@@ -806,11 +815,11 @@ bool fp_rows_fits(int cols, int nt) { return fp_rows_slots(cols, nt) > 0; }
 template <int MODE>
 static cudaError_t launch_bp_rows_t(const BpArgs &a, const float *rows, int cols, cudaStream_t s) {
   const int stages = bp_rows_stages(cols, a.nt);
-  const size_t smem = std::max<size_t>(bp_rows_smem(cols, a.nt, stages), kRowTile * 512);
+  const size_t smem = std::max<size_t>(bp_rows_smem(cols, a.nt, stages), kRowTile * kBpQuads * 16);
   cudaError_t e = cudaFuncSetAttribute(bp_rows_kernel<MODE>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  const dim3 grid((a.v.nx + kBpX - 1) / kBpX, (a.v.nz + kBpZ - 1) / kBpZ,
+  const dim3 grid((a.v.nx + kRowBpX - 1) / kRowBpX, (a.v.nz + kRowBpZ - 1) / kRowBpZ,
                   (a.v.ny + kRowTile - 1) / kRowTile);
   bp_rows_kernel<MODE><<<grid, kBpWarps * 32, smem, s>>>(a, rows, cols, stages);
   return cudaGetLastError();
@@ -828,9 +837,9 @@ cudaError_t launch_fp_rows(const FpArgs &a, float *rows, int cols, int nsm, cuda
   cudaError_t e = cudaFuncSetAttribute(fp_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem);
   if (e != cudaSuccess) return e;
-  const dim3 grid((a.v.nx + kFpX - 1) / kFpX, (a.v.nz + kFpZ - 1) / kFpZ,
+  const dim3 grid((a.v.nx + kRowFpX - 1) / kRowFpX, (a.v.nz + kRowFpZ - 1) / kRowFpZ,
                   (a.v.ny + kRowTile - 1) / kRowTile);
-  fp_rows_kernel<<<grid, kFpWarps * 32, smem, s>>>(a, rows, cols, slots, smem <= kRowSmem2 ? 2 * nsm : nsm);
+  fp_rows_kernel<<<grid, kFpWarps * 32, smem, s>>>(a, rows, cols, slots, smem <= kRowSmem / kFpPerSm ? kFpPerSm * nsm : nsm);
   return cudaGetLastError();
 }
 
