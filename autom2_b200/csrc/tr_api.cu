@@ -386,6 +386,34 @@ tr_status run_fp(tr_ctx *c, const FpArgs &a, cudaStream_t s) {
   return TR_OK;
 }
 
+void set_weights(const tr_ctx *c, BpArgs *b);
+
+// One SIRT iteration over the whole volume with FP32 residuals on the row-
+// invariant path, the residual formed between the row stacks: *done says
+// whether it ran (else nothing was launched).
+tr_status sirt_rows(tr_ctx *c, const void *proj, int pdtype, const float *ps, float *vol,
+                    float gamma, cudaStream_t s, bool *done) {
+  const size_t sums = row_stack_floats(c->nx, c->ny, c->nt, c->rfp_cols) * sizeof(float);
+  *done = !c->deterministic && rows_path(c, kRowsBp, c->th, c->nt, s) &&
+          rows_path(c, kRowsFp, c->th, c->nt, s) && bp_rows_fits(c->rbp_cols, c->nt) &&
+          fp_rows_fits(c->rfp_cols, c->nt) && scratch_try(c, (void **)&c->rowsum_d, sums) &&
+          scratch_try(c, (void **)&c->rows_d,
+                      row_stack_floats(c->nx, c->ny, c->nt, c->rbp_cols) * sizeof(float));
+  if (!*done) return TR_OK;
+  TR_CUDA(c, rows_acquire(c, s));
+  TR_CUDA(c, cudaMemsetAsync(c->err_d, 0, sizeof(int), s));
+  TR_CUDA(c, cudaMemsetAsync(c->rowsum_d, 0, sums, s));
+  TR_CUDA(c, launch_fp_rows(fp_args(c, vol, 0, c->th, nullptr, 0, c->nt), c->rowsum_d, c->rfp_cols,
+                            c->nsm, s));
+  TR_CUDA(c, launch_resid_rows(c->rowsum_d, c->rfp_cols, proj, pdtype, ps, c->wt_d, c->geo_d, c->nt,
+                               c->oy, c->nx, c->ny, c->rows_d, c->rbp_cols, s));
+  BpArgs b = bp_args(c, vol, 0, c->th, nullptr, 0, c->nt, gamma);
+  set_weights(c, &b);
+  TR_CUDA(c, launch_bp_rows(BP_SIRT, b, c->rows_d, c->rbp_cols, s));
+  TR_CUDA(c, rows_release(c, s));
+  return TR_OK;
+}
+
 // Kernel spectrum of the R-weighting filter for rows of nx samples.
 tr_status build_filter(tr_ctx *c, int nx) {
   if (c->filt_nx == nx && c->ghat_d && c->tw_d) {  // cached: claim for this problem
@@ -1027,6 +1055,9 @@ tr_status tr_sirt(tr_ctx *c, const float *proj, float *vol, int iters, float gam
   if ((st = ensure_wt(c, s))) return st;
   if ((st = ensure_wtvol(c, 0, c->th, s))) return st;
   for (int it = 0; it < iters; ++it) {
+    bool done = false;
+    TR_TRY(sirt_rows(c, proj, TR_DTYPE_F32, nullptr, vol, gamma, s, &done));
+    if (done) continue;
     TR_CUDA(c, cudaMemsetAsync(c->val_d, 0, pn * sizeof(float), s));
     FpArgs f = fp_args(c, vol, 0, c->th, c->val_d, 0, c->nt);
     TR_TRY(run_fp(c, f, s));
@@ -1159,6 +1190,9 @@ tr_status tr_sirt_lp(tr_ctx *c, const void *proj, int pdtype, const float *scale
   void *res = rdtype == TR_DTYPE_F32 ? (void *)c->val_d : c->res16_d;
   const float *rs = rdtype == TR_DTYPE_F16 ? c->rscale_d : nullptr;
   for (int it = 0; it < iters; ++it) {
+    bool done = false;
+    if (rdtype == TR_DTYPE_F32) TR_TRY(sirt_rows(c, proj, pdtype, ps, vol, gamma, s, &done));
+    if (done) continue;
     TR_CUDA(c, cudaMemsetAsync(c->val_d, 0, pn * sizeof(float), s));
     FpArgs f = fp_args(c, vol, 0, c->th, c->val_d, 0, c->nt);
     TR_TRY(run_fp(c, f, s));

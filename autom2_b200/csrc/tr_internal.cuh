@@ -272,6 +272,11 @@ cudaError_t launch_fp_rows(const FpArgs &a, float *rows, int cols, int nsm, cuda
 cudaError_t launch_unblend_rows(const float *rows, const TiltGeo *geo, int t0, int nt, float oy,
                                 int vny, int margin, float *val, long long tstride, int nx, int ny,
                                 cudaStream_t s);
+// The residual p ps - val/wt of all nt tilts from the forward projection's row
+// sums (margin smargin), as the row stack (margin `margin`) of a BP_SIRT.
+cudaError_t launch_resid_rows(const float *sums, int smargin, const void *p, int pdtype,
+                              const float *ps, const float *wt, const TiltGeo *geo, int nt, float oy,
+                              int nx, int ny, float *rows, int margin, cudaStream_t s);
 cudaError_t launch_resid(const float *p, float *val, const float *wt, size_t n, int nsm,
                          cudaStream_t s);
 cudaError_t launch_quantize(const float *p, size_t plane, int nt, int dtype, void *out,

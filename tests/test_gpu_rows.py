@@ -70,7 +70,15 @@ def test_sirt_and_a_slab_of_sections(engine, restatement, nx, ny, nt, th, layout
     engine.set_problem(nx, ny, nt, th, c8, layout, org)
     v = torch.from_numpy(vol).cuda()
     engine.sirt(torch.from_numpy(proj).cuda(), v, 2, 0.5)
-    assert O.rel_l2(v.cpu().numpy(), R.sirt(g, c8, proj, vol, 2, 0.5, fp64=True)) < TOL
+    want = R.sirt(g, c8, proj, vol, 2, 0.5, fp64=True)
+    assert O.rel_l2(v.cpu().numpy(), want) < TOL
+    # a stack that 16 bits hold exactly, FP32 residuals: the same iteration
+    whole16 = np.round(proj * 8)
+    for dtype in (torch.float16, torch.bfloat16):
+        q, scale = engine.quantize(torch.from_numpy(whole16).cuda(), dtype)
+        v = torch.from_numpy(vol).cuda()
+        engine.sirt_lp(q, scale, v, 2, 0.5, "f32")
+        assert O.rel_l2(v.cpu().numpy(), R.sirt(g, c8, whole16, vol, 2, 0.5, fp64=True)) < TOL
     # sections [z0, z0 + nz) alone: the same voxels as the whole volume's
     z0, nz = 5, th - 9
     whole = torch.zeros(vol.shape, device="cuda")
