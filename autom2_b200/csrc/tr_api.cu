@@ -1119,16 +1119,34 @@ tr_status tr_sart(tr_ctx *c, const float *proj, float *vol, int iters, float gam
                           "reprojection")))
     return st;
   if ((st = ensure_wt(c, s))) return st;
-  for (int it = 0; it < iters; ++it)
-    for (int t = 0; t < c->nt; ++t) {
-      float *vt = c->val_d + plane * t;
+  const int steps = iters * c->nt;
+  for (int i = 0; i < steps; ++i) {
+    const int t = i % c->nt;
+    float *vt = c->val_d + plane * t;
+    // The volume's projection at the first tilt; later ones come with the update
+    // of the tilt before (the deterministic flush has no such form).
+    if (i == 0 || c->deterministic) {
       TR_CUDA(c, cudaMemsetAsync(vt, 0, plane * sizeof(float), s));
-      FpArgs f = fp_args(c, vol, 0, c->th, c->val_d, t, 1);
-      TR_TRY(run_fp(c, f, s));
-      TR_CUDA(c, launch_resid(proj + plane * t, vt, c->wt_d + plane * t, plane, c->nsm, s));
-      BpArgs b = bp_args(c, vol, 0, c->th, c->val_d, t, 1, gamma);
-      TR_CUDA(c, run_bp(c, BP_NORM, b, s));
+      TR_TRY(run_fp(c, fp_args(c, vol, 0, c->th, c->val_d, t, 1), s));
     }
+    TR_CUDA(c, launch_resid(proj + plane * t, vt, c->wt_d + plane * t, plane, c->nsm, s));
+    if (i + 1 < steps && !c->deterministic && c->nt > 1) {
+      const int n = (i + 1) % c->nt;
+      TR_CUDA(c, cudaMemsetAsync(c->val_d + plane * n, 0, plane * sizeof(float), s));
+      FpArgs f = fp_args(c, vol, 0, c->th, c->val_d, n, 1);
+      f.chunk = 1;
+      f.simg = vt;
+      f.sgeo = c->geo_d + t;
+      f.sgamma = gamma;
+      TR_CUDA(c, launch_sart_sweep(c->sep, f, s));
+    } else {
+      TR_CUDA(c, run_bp(c, BP_NORM, bp_args(c, vol, 0, c->th, c->val_d, t, 1, gamma), s));
+      if (i + 1 < steps && !c->deterministic) {  // a single tilt: its residual plane is in use
+        TR_CUDA(c, cudaMemsetAsync(vt, 0, plane * sizeof(float), s));
+        TR_TRY(run_fp(c, fp_args(c, vol, 0, c->th, c->val_d, t, 1), s));
+      }
+    }
+  }
   return TR_OK;
 }
 

@@ -120,6 +120,12 @@ struct FpArgs {
   const unsigned *gmax;
   double gbound;
   int *err;           // row-invariant path: as BpArgs::err
+  // SART sweep (simg != nullptr): the voxels are first updated from the residual
+  // plane simg ([pny][pnx]) of the tilt with geometry sgeo, v += sgamma s/c, and
+  // written back; the updated ones are projected.
+  const float *simg;
+  const TiltGeo *sgeo;
+  float sgamma;
 };
 
 // Footprint bookkeeping of one tilt for one tile, computed in FP64.
@@ -243,6 +249,9 @@ cudaError_t launch_classify_tiles(const TiltGeo *geo, int nt, const VolView &v, 
 cudaError_t launch_sep_row_weights(const TiltGeo *geo, int nt, int ny, float oy, int pny,
                                    float *wrow, cudaStream_t s);
 cudaError_t launch_fp(bool sep, const FpArgs &a, cudaStream_t s);
+// The back-projection update of one tilt and the forward projection of another
+// in one pass over the volume (FpArgs::simg).
+cudaError_t launch_sart_sweep(bool sep, const FpArgs &a, cudaStream_t s);
 // Deterministic forward projection into a.val: the view's max |voxel| into
 // *gmax, the splat with the int64 flush into ival (all zero on entry, left
 // zero), then the sums converted and added into a.val.

@@ -790,7 +790,84 @@ struct FpShared {
   int nonzero;
 };
 
-template <bool SEP, bool DET = false>
+// s/c of the reference's normalised back-projection (BackProject, main-mpi.cpp:
+// 411-450) for a lower neighbour (k, j) and fractions fu, fv: the edge-clamped
+// image's bilinear value where that neighbour lies in [-1, nx-1] x [-1, ny-1],
+// nothing elsewhere.  INSIDE: all four taps are in the image.
+template <bool INSIDE>
+__device__ __forceinline__ float gather_normalised(const float *__restrict__ img, int nx, int ny,
+                                                   int k, int j, float fu, float fv) {
+  float p00, p01, p10, p11;
+  if (INSIDE) {
+    const float *p = img + (size_t)j * nx + k;
+    p00 = __ldg(p), p01 = __ldg(p + 1), p10 = __ldg(p + nx), p11 = __ldg(p + nx + 1);
+  } else {
+    if (k < -1 || k > nx - 1 || j < -1 || j > ny - 1) return 0.f;
+    const int k0 = max(k, 0), k1 = min(k + 1, nx - 1);
+    const float *p = img + (size_t)max(j, 0) * nx, *q = img + (size_t)min(j + 1, ny - 1) * nx;
+    p00 = __ldg(p + k0), p01 = __ldg(p + k1), p10 = __ldg(q + k0), p11 = __ldg(q + k1);
+  }
+  const float r0 = fmaf(fu, p01 - p00, p00), r1 = fmaf(fu, p11 - p10, p10);
+  return fmaf(fv, r1 - r0, r0);
+}
+
+// The update of a SART sweep: the thread's voxel pairs (FpArgs::simg), read,
+// updated and written back.
+template <bool INSIDE>
+__device__ __forceinline__ void sart_update_pairs(const FpArgs &a, const TileTilt &tt,
+                                                  const TiltGeo &g, int x, int y, int z0, int lane,
+                                                  int wy, int wz, float (&va)[kFNV],
+                                                  float (&vb)[kFNV]) {
+  const long long A0 = g.A[0], A2 = g.A[2], B0 = g.B[0], B2 = g.B[2];
+  unsigned long long U = (unsigned long long)(tt.U0 + wy * g.A[1] + (long long)(wz * kFNV) * A2 +
+                                              (2 * lane) * A0);
+  unsigned long long V = (unsigned long long)(tt.V0 + wy * g.B[1] + (long long)(wz * kFNV) * B2 +
+                                              (2 * lane) * B0);
+  const bool ina = x < a.v.nx && y < a.v.ny, inb = x + 1 < a.v.nx && y < a.v.ny;
+  float *p = a.v.vol + (size_t)y * a.v.sy + (size_t)z0 * a.v.sz + x;
+  const bool pair = inb && ((a.v.sy | a.v.sz) & 1) == 0 &&
+                    (reinterpret_cast<uintptr_t>(a.v.vol) & 7) == 0;
+#pragma unroll
+  for (int k = 0; k < kFNV; ++k) {
+    const bool inz = z0 + k < a.v.nz;
+    float2 v = make_float2(0.f, 0.f);
+    if (inz && pair) v = *reinterpret_cast<const float2 *>(p + (size_t)k * a.v.sz);
+    else if (inz) {
+      if (ina) v.x = p[(size_t)k * a.v.sz];
+      if (inb) v.y = p[(size_t)k * a.v.sz + 1];
+    }
+    va[k] = v.x;
+    vb[k] = v.y;
+  }
+#pragma unroll
+  for (int k = 0; k < kFNV; ++k) {
+    const bool inz = z0 + k < a.v.nz;
+    if (inz && ina)
+      va[k] += a.sgamma * gather_normalised<INSIDE>(a.simg, a.pnx, a.pny, tt.kmin + (int)(U >> 32),
+                                                    tt.jmin + (int)(V >> 32),
+                                                    one_plus_frac(U) - 1.f, one_plus_frac(V) - 1.f);
+    const unsigned long long Ub = U + A0, Vb = V + B0;
+    if (inz && inb)
+      vb[k] += a.sgamma * gather_normalised<INSIDE>(a.simg, a.pnx, a.pny, tt.kmin + (int)(Ub >> 32),
+                                                    tt.jmin + (int)(Vb >> 32),
+                                                    one_plus_frac(Ub) - 1.f,
+                                                    one_plus_frac(Vb) - 1.f);
+    U += (unsigned long long)A2;
+    V += (unsigned long long)B2;
+  }
+#pragma unroll
+  for (int k = 0; k < kFNV; ++k) {
+    if (z0 + k >= a.v.nz) continue;
+    float *q = p + (size_t)k * a.v.sz;
+    if (pair) *reinterpret_cast<float2 *>(q) = make_float2(va[k], vb[k]);
+    else {
+      if (ina) q[0] = va[k];
+      if (inb) q[1] = vb[k];
+    }
+  }
+}
+
+template <bool SEP, bool DET = false, bool SART = false>
 __device__ __forceinline__ void fp_tile(const FpArgs &a, int bx, int by, int bz,
                                         float *accs, FpShared &sh) {
   TileTilt *const tt = sh.tt;
@@ -811,7 +888,19 @@ __device__ __forceinline__ void fp_tile(const FpArgs &a, int bx, int by, int bz,
   const int per = fh * fw;
 
   float va[kFNV], vb[kFNV];
-  {
+  if constexpr (SART) {
+    if (tid == 0)
+      tile_setup(*a.sgeo, xc, yc, zc, a.ox, a.oy, a.oz, a.pny, false, kFX - 1, kTY - 1, kFTZ - 1,
+                 tt[0], sw[0]);
+    __syncthreads();
+    const TileTilt t0 = tt[0];
+    // the window holds every lower neighbour, its upper one and a margin of one
+    const bool inside = t0.kmin >= 0 && t0.kmin + t0.nq <= a.pnx && t0.jmin >= 0 &&
+                        t0.jmin + t0.nr <= a.pny;
+    const int x = xc + 2 * lane, y = yc + wy, z0 = zl + wz * kFNV;
+    if (inside) sart_update_pairs<true>(a, t0, *a.sgeo, x, y, z0, lane, wy, wz, va, vb);
+    else sart_update_pairs<false>(a, t0, *a.sgeo, x, y, z0, lane, wy, wz, va, vb);
+  } else {
     const int x = xc + 2 * lane, y = yc + wy;
     const bool ina = x < a.v.nx && y < a.v.ny, inb = x + 1 < a.v.nx && y < a.v.ny;
 #pragma unroll
@@ -1022,6 +1111,18 @@ __device__ __forceinline__ void fp_tile(const FpArgs &a, int bx, int by, int bz,
 
     __syncthreads();
   }
+}
+
+// SART's step from one tilt to the next in one pass over the volume: read,
+// update from the residual of the tilt before, write, splat for the tilt after.
+// Taps come straight from the residual plane (a few MB, in L2): a table would be
+// used once.  61 tilts of 512 x 512 on 128 sections, per tilt: TODO us from 157
+// (a forward projection and a back-projection, which read the volume twice).
+template <bool SEP>
+__global__ void __launch_bounds__(kThreads, 3) sart_sweep_kernel(const FpArgs a) {
+  extern __shared__ __align__(16) float accs[];
+  __shared__ FpShared sh;
+  fp_tile<SEP, false, true>(a, blockIdx.x, blockIdx.y, blockIdx.z, accs, sh);
 }
 
 template <bool SEP, bool DET>
@@ -1644,6 +1745,20 @@ cudaError_t launch_fp(bool sep, const FpArgs &a, cudaStream_t s) {
   if (a.ival)
     return sep ? launch_fp_t<true, true>(a, smem, s) : launch_fp_t<false, true>(a, smem, s);
   return sep ? launch_fp_t<true, false>(a, smem, s) : launch_fp_t<false, false>(a, smem, s);
+}
+
+template <bool SEP>
+static cudaError_t launch_sart_t(const FpArgs &a, size_t smem, cudaStream_t s) {
+  cudaError_t e = cudaFuncSetAttribute(sart_sweep_kernel<SEP>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  sart_sweep_kernel<SEP><<<fp_grid(a.v), kThreads, smem, s>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_sart_sweep(bool sep, const FpArgs &a, cudaStream_t s) {
+  const size_t smem = (size_t)a.chunk * (sep ? kTY : a.fh) * a.fw * sizeof(float);
+  return sep ? launch_sart_t<true>(a, smem, s) : launch_sart_t<false>(a, smem, s);
 }
 
 // Largest |voxel| of a view, as float bits, max-combined into *out (which
