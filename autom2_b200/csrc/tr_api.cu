@@ -94,7 +94,7 @@ struct tr_ctx {
   unsigned *gmax_d = nullptr;
   // row-invariant geometries: the back-projection's voxel-row stack and the
   // forward projection's row sums, and the last use of either
-  bool rows = false;
+  bool rows = false, product_weights = false;
   int rbp_cols = 0, rfp_cols = 0;
   float *rows_d = nullptr, *rowsum_d = nullptr;
   cudaEvent_t ev_rows = nullptr;
@@ -388,6 +388,19 @@ tr_status run_fp(tr_ctx *c, const FpArgs &a, cudaStream_t s) {
 
 void set_weights(const tr_ctx *c, BpArgs *b);
 
+// Projection weights of sections [z0, z0 + nz) and tilts [t0, t0 + nt), plane t0
+// at wt, added to what is there.
+tr_status run_weights(tr_ctx *c, int z0, int nz, int t0, int nt, float *wt, cudaStream_t s) {
+  if (c->product_weights) {
+    TR_CUDA(c, launch_weight_rows(c->geo_d + t0, nt, c->nx, c->ny, z0, nz, c->ox, c->oy, c->oz, wt,
+                                  (long long)c->nx * c->ny, true, s));
+    return TR_OK;
+  }
+  FpArgs w = fp_args(c, nullptr, z0, nz, wt, 0, nt);
+  w.geo = c->geo_d + t0;
+  return run_fp(c, w, s);
+}
+
 // One SIRT iteration over the whole volume with FP32 residuals on the row-
 // invariant path, the residual formed between the row stacks: *done says
 // whether it ran (else nothing was launched).
@@ -480,6 +493,7 @@ tr_status load_geometry(tr_ctx *c, const double *coeff8, cudaStream_t s) {
   c->fp_nbound = gi.nbound;
   c->sep = gi.sep;
   c->rows = gi.rows;
+  c->product_weights = gi.product_weights;
   c->rbp_cols = gi.rbp_cols;
   c->rfp_cols = gi.rfp_cols;
   c->chunk_bp = chunk_for(kSmemBp, gi.bp_tilt_bytes);
@@ -507,14 +521,20 @@ tr_status need_problem(tr_ctx *c) {
   return TR_OK;
 }
 
+tr_status run_weights(tr_ctx *c, int z0, int nz, int t0, int nt, float *wt, cudaStream_t s);
+
 tr_status ensure_wt(tr_ctx *c, cudaStream_t s) {
   const size_t pb = proj_elems(c) * sizeof(float);
   tr_status st = scratch_alloc(c, (void **)&c->wt_d, pb, "projection weights");
   if (st) return st;
   if (!c->wt_ready) {
-    TR_CUDA(c, cudaMemsetAsync(c->wt_d, 0, pb, s));
-    FpArgs a = fp_args(c, nullptr, 0, c->th, c->wt_d, 0, c->nt);
-    if ((st = run_fp(c, a, s))) return st;
+    if (c->product_weights) {
+      TR_CUDA(c, launch_weight_rows(c->geo_d, c->nt, c->nx, c->ny, 0, c->th, c->ox, c->oy, c->oz,
+                                    c->wt_d, (long long)c->nx * c->ny, false, s));
+    } else {
+      TR_CUDA(c, cudaMemsetAsync(c->wt_d, 0, pb, s));
+      if ((st = run_weights(c, 0, c->th, 0, c->nt, c->wt_d, s))) return st;
+    }
     c->wt_ready = true;
   }
   return TR_OK;
@@ -979,10 +999,7 @@ tr_status tr_forward_project(tr_ctx *c, const float *vol, int z0, int nz, float 
     return fail(c, TR_ERR_ARG, "bad forward-projection arguments (z0=%d nz=%d)", z0, nz);
   FpArgs a = fp_args(c, vol, z0, nz, val, 0, c->nt);
   TR_TRY(run_fp(c, a, (cudaStream_t)stream));
-  if (wt) {
-    FpArgs w = fp_args(c, nullptr, z0, nz, wt, 0, c->nt);
-    TR_TRY(run_fp(c, w, (cudaStream_t)stream));
-  }
+  if (wt) TR_TRY(run_weights(c, z0, nz, 0, c->nt, wt, (cudaStream_t)stream));
   return TR_OK;
 }
 
@@ -997,11 +1014,7 @@ tr_status tr_forward_project_tilts(tr_ctx *c, const float *vol, int z0, int nz, 
   FpArgs a = fp_args(c, vol, z0, nz, val, 0, ntilts);
   a.geo = c->geo_d + t0;
   TR_TRY(run_fp(c, a, (cudaStream_t)stream));
-  if (wt) {
-    FpArgs w = fp_args(c, nullptr, z0, nz, wt, 0, ntilts);
-    w.geo = c->geo_d + t0;
-    TR_TRY(run_fp(c, w, (cudaStream_t)stream));
-  }
+  if (wt) TR_TRY(run_weights(c, z0, nz, t0, ntilts, wt, (cudaStream_t)stream));
   return TR_OK;
 }
 

@@ -17,6 +17,7 @@ struct GeomInfo {
   float nbound;    // most voxel contributions one forward window entry collects
   bool sep;        // every tilt has b1 = b3 = 0, b2 = 1 (separable rows)
   bool rows;       // row-invariant: every tilt has a2 = 0, 0 <= a1 <= 1, |a3| <= 1, and sep
+  bool product_weights;  // sep, a2 = 0 and |a1| >= 0.05: weight = column's times row's
   int rbp_cols, rfp_cols;  // window columns of a row-invariant tile (tr_rows.cu)
   size_t fp_tilt_bytes;  // shared memory of one staged tilt's splat window
   size_t bp_tilt_bytes;  // shared memory of one staged tilt's interpolation table
@@ -72,7 +73,7 @@ constexpr int kRowFpX = 16, kRowFpZ = 4;
 // offending tilt for the per-tilt failures.
 inline int derive_geometry(const double *coeff8, int nt, int nx, int ny, int th,
                            size_t smem_max, TiltGeo *g, GeomInfo *out, int *bad_tilt) {
-  bool sep = true, rows = true;
+  bool sep = true, rows = true, product = true;
   double rbp = 0, rfp = 0;
   double span_u = 0, span_v = 0, fspan_u = 0, fspan_v = 0, min_a1 = 1e30, sect = 0;
   const double two32 = 4294967296.0;
@@ -100,6 +101,7 @@ inline int derive_geometry(const double *coeff8, int nt, int nx, int ny, int th,
     if (reach_u > 1.0e9 || reach_v > 1.0e9) return GEOM_RANGE;
     if (!(k[5] == 0.0 && k[7] == 0.0 && k[6] == 1.0)) sep = false;
     if (!(k[2] == 0.0 && k[1] >= 0.0 && k[1] <= 1.0 && std::fabs(k[3]) <= 1.0)) rows = false;
+    if (!(k[2] == 0.0 && std::fabs(k[1]) >= 0.05)) product = false;
     rbp = std::max(rbp, std::fabs(k[1]) * (kRowBpX - 1) + std::fabs(k[3]) * (kRowBpZ - 1));
     rfp = std::max(rfp, std::fabs(k[1]) * (kRowFpX - 1) + std::fabs(k[3]) * (kRowFpZ - 1));
     min_a1 = std::min(min_a1, std::fabs(k[1]));
@@ -133,6 +135,7 @@ inline int derive_geometry(const double *coeff8, int nt, int nx, int ny, int th,
   // reach lower columns up to floor(umax) and one more for the fixed-point
   // coordinates, and the column above.
   out->rows = sep && rows;
+  out->product_weights = sep && product;
   out->rbp_cols = (int)std::ceil(rbp) + 4;
   out->rfp_cols = (int)std::ceil(rfp) + 4;
   out->fp_tilt_bytes = (size_t)out->ffw * out->ffh * sizeof(int);

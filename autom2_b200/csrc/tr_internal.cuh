@@ -281,6 +281,11 @@ cudaError_t launch_fp_rows(const FpArgs &a, float *rows, int cols, int nsm, cuda
 cudaError_t launch_unblend_rows(const float *rows, const TiltGeo *geo, int t0, int nt, float oy,
                                 int vny, int margin, float *val, long long tstride, int nx, int ny,
                                 cudaStream_t s);
+// Projection weights of sections [z0, z0 + nz) where GeomInfo::product_weights
+// (tilts geo[0..nt), planes wt + t tstride): written, or added.
+cudaError_t launch_weight_rows(const TiltGeo *geo, int nt, int nx, int ny, int z0, int nz, float ox,
+                               float oy, float oz, float *wt, long long tstride, bool add,
+                               cudaStream_t s);
 // The residual p ps - val/wt of all nt tilts from the forward projection's row
 // sums (margin smargin), as the row stack (margin `margin`) of a BP_SIRT.
 cudaError_t launch_resid_rows(const float *sums, int smargin, const void *p, int pdtype,

@@ -854,6 +854,62 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// Projection weights (the splat of ones) of separable geometries whose columns
+// do not depend on the row (a2 = 0): the weight of detector pixel (j, k) is a
+// column's times a row's,
+//   sum over x, z of the tent 1 - |u(x, z) - k|  times  sum over y of 1 - |v(y) - j|,
+// so a block sums its tilt's 32 columns in FP64 (the few x per section that
+// reach them, |a1| being 0.05 or more) and writes all their pixels.  61 tilts of
+// 2048 x 2048, 128 sections: 12.2 ms as a forward projection of ones -> 0.26 ms.
+template <bool ADD>
+__global__ void __launch_bounds__(256)
+    weight_rows_kernel(const TiltGeo *__restrict__ geo, int nx, int ny, int z0, int nz, float ox,
+                       float oy, float oz, float *__restrict__ wt, long long tstride) {
+  __shared__ double part[8][32];
+  const int t = blockIdx.y, lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int k = blockIdx.x * 32 + lane;
+  const TiltGeo &g = geo[t];
+  const double a1 = g.a[1], inv = 1.0 / a1, reach = fabs(inv);
+  double sum = 0.0;
+  for (int z = wp; z < nz; z += 8) {
+    const double c = g.a[0] + g.a[3] * (double)((float)(z0 + z) - oz) + (double)ox - (double)k;
+    const double xm = (double)ox - c * inv;  // where u = k
+    const int x0 = max(0, (int)floor(xm - reach)), x1 = min(nx - 1, (int)ceil(xm + reach));
+    for (int x = x0; x <= x1; ++x)
+      sum += fmax(0.0, 1.0 - fabs(c + a1 * (double)((float)x - ox)));
+  }
+  part[wp][lane] = sum;
+  __syncthreads();
+  double all = 0.0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) all += part[w][lane];
+  const float cw = (float)all;
+  const int S = (int)floor(g.b[0]);
+  float *p = wt + (size_t)t * tstride + k;
+  for (int j0 = wp * 32; j0 < ny; j0 += 256) {
+    // lane: the row weight of detector row j0 + lane, from the voxel rows that
+    // can reach it
+    const int j = j0 + lane;
+    float rw = 0.f;
+#pragma unroll
+    for (int h = -2; h <= 1; ++h) {
+      const int y = j - S + h;
+      if (y < 0 || y >= ny) continue;
+      float dy;
+      const int y0 = voxel_row(g, y, oy, dy);
+      if (y0 == j) rw += 1 - dy;
+      else if (y0 == j - 1) rw += dy;
+    }
+    for (int i = 0; i < min(32, ny - j0); ++i) {
+      const float r = __shfl_sync(0xffffffffu, rw, i);
+      if (k < nx) {
+        float *q = p + (size_t)(j0 + i) * nx;
+        *q = ADD ? *q + cw * r : cw * r;
+      }
+    }
+  }
+}
+
 }  // namespace
 
 // ------------------------------------------------------------ launchers
@@ -898,6 +954,20 @@ cudaError_t launch_resid_rows(const float *sums, int smargin, const void *p, int
   else
     resid_rows_kernel<<<grid, 256, 0, s>>>(sums, smargin, (const float *)p, ps, wt, geo, oy, nx, ny,
                                            rows, margin);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_weight_rows(const TiltGeo *geo, int nt, int nx, int ny, int z0, int nz, float ox,
+                               float oy, float oz, float *wt, long long tstride, bool add,
+                               cudaStream_t s) {
+  for (int t = 0; t < nt; t += 65535) {
+    const dim3 grid((nx + 31) / 32, std::min(65535, nt - t));
+    float *w = wt + (size_t)t * tstride;
+    if (add)
+      weight_rows_kernel<true><<<grid, 256, 0, s>>>(geo + t, nx, ny, z0, nz, ox, oy, oz, w, tstride);
+    else
+      weight_rows_kernel<false><<<grid, 256, 0, s>>>(geo + t, nx, ny, z0, nz, ox, oy, oz, w, tstride);
+  }
   return cudaGetLastError();
 }
 

@@ -343,8 +343,13 @@ tr_status admit(tr_sched *S, Job &j) {
   // tiles' slots come from a device counter, so the worst-case buffer needs
   // no read-back of the count).
   if (sirt) {
-    SCHED_CUDA(S, cudaMemsetAsync(j.wt, 0, P * 4, ps));
-    SCHED_CUDA(S, launch_fp(j.gi.sep, job_fp(S, j, nullptr, j.wt), ps));
+    if (j.gi.product_weights) {
+      SCHED_CUDA(S, launch_weight_rows(j.geo, nt, j.d.nx, j.d.ny, 0, j.d.thickness, j.d.ox, j.d.oy,
+                                       j.d.oz, j.wt, (long long)j.d.nx * j.d.ny, false, ps));
+    } else {
+      SCHED_CUDA(S, cudaMemsetAsync(j.wt, 0, P * 4, ps));
+      SCHED_CUDA(S, launch_fp(j.gi.sep, job_fp(S, j, nullptr, j.wt), ps));
+    }
     SCHED_CUDA(S, cudaMemsetAsync(j.wslot + tiles, 0, sizeof(int), ps));
     SCHED_CUDA(S, launch_classify_tiles(j.geo, nt, job_view(j, nullptr), j.d.ox, j.d.oy, j.d.oz,
                                         j.d.nx, j.d.ny, j.gi.sep, j.wslot, j.wslot + tiles, ps));
