@@ -258,29 +258,38 @@ BpArgs bp_args(const tr_ctx *c, float *vol, int z0, int nz, const float *img,
 }
 
 // Row-invariant path (tr_rows.cu) for a launch over nz sections and nt tilts on
-// `s`.  Its tiles are 16 x 128 x 8 voxels where the general kernels' are
-// (general_x) x 4 x 32, so it takes the launches whose padding to its tiles
-// (most of all of the rows to 128) does not outweigh its gain -- `pad` bounds
-// the padded voxels relative to the general kernels' -- and which have tiles
-// enough for the SMs.  Measured (us, general / row-invariant):
+// `s`.  Its tiles are 16 x 128 x 8 voxels (16 x 128 x 4 in the projection and
+// for 16-bit stacks) where the general kernels' are (general_x) x 4 x 32, so it
+// takes the launches whose padding to its tiles (most of all of the rows to 128)
+// does not outweigh its gain -- `pad` bounds the padded voxels relative to the
+// general kernels' -- and which have tiles (counted 8 sections deep) enough for
+// the SMs.  Measured (us, general / row-invariant):
 //   back-projection, pad 1.35, 128 tiles: 1024 x 1024 x 256, 61 tilts 6686 /
 //     3833; x 64, 1 tilt 320 / 147; 256 x 256 x 64, 41 tilts 91 / 68; rows 192
 //     of 256 (pad 1.33) 182 / 165, 160 of 256 (1.6) 110 / 116; 256 x 64 x 64
 //     (64 tiles, pad 2) 37 / 48;
+//   of 16-bit stacks (compensated sums; the general kernel reads the 16 bits,
+//     the row stack is FP32 and its blend must be shared by sections enough),
+//     pad 1.1, 32 tilts, 96 sections: 1024 x 1024 x 256, 61 tilts 6905 / 6172,
+//     x 64, 24 tilts 762 / 780; 256 x 256 x 64, 41 tilts 91 / 97; 512 x 200 x 64
+//     (pad 1.28) 130 / 166; 1024 x 1024 x 64, 8 tilts (pad 1) 330 / 356.  Any
+//     such stack where the general kernel is the one to pad (0.85): 250 x 250 x
+//     66, 41 tilts (0.77) 161 / 103; 1000 x 1000 x 100 (0.84) 2367 / 1793;
 //   forward projection, pad 1.15, 256 tiles: 1024 x 1024 x 256, 61 tilts 8123 /
-//     6071; x 64: 41 tilts 1408 / 1280, 24 tilts 820 / 826, 8 tilts 305 / 459
+//     5742; x 64: 41 tilts 1408 / 1280, 24 tilts 820 / 774, 8 tilts 305 / 459
 //     (the tilts pass through a CTA's warps in a pipeline that must fill);
-//     256 x 256 x 64 125 / 100, x 32 (128 tiles) 99 / 112; rows 320 of 384
+//     256 x 256 x 64 125 / 98, x 32 (128 tiles) 99 / 112; rows 320 of 384
 //     (pad 1.2) 355 / 391.
 // Not under stream capture, whose graphs must not hold a buffer that the
 // context may drop.
 struct RowsRule {
-  int general_x, min_tilts, min_tiles;
+  int general_x, min_tilts, min_tiles, min_z;
   double pad;
 };
-constexpr RowsRule kRowsBp{kTX, 1, 128, 1.35}, kRowsFp{kFX, 24, 256, 1.15};
+constexpr RowsRule kRowsBp{kTX, 1, 128, 1, 1.35}, kRowsBp16{kTX, 32, 128, 96, 1.1},
+    kRowsBp16Pad{kTX, 1, 128, 1, 0.85}, kRowsFp{kFX, 24, 256, 1, 1.15};
 bool rows_path(const tr_ctx *c, const RowsRule &r, int nz, int nt, cudaStream_t s) {
-  if (!c->rows || nt < r.min_tilts) return false;
+  if (!c->rows || nt < r.min_tilts || nz < r.min_z) return false;
   const auto tiles = [](int n, int t) { return (double)((n + t - 1) / t); };
   const double n = tiles(c->nx, kRowBpX) * tiles(c->ny, kRowTile) * tiles(nz, kRowBpZ);
   const double general = tiles(c->nx, r.general_x) * r.general_x * tiles(c->ny, kTY) * kTY *
@@ -306,14 +315,18 @@ cudaError_t rows_release(tr_ctx *c, cudaStream_t s) { return cudaEventRecord(c->
 cudaError_t run_bp(tr_ctx *c, int mode, const BpArgs &a, cudaStream_t s) {
   cudaError_t e;
   if (c->err_d && (e = cudaMemsetAsync(c->err_d, 0, sizeof(int), s)) != cudaSuccess) return e;
-  if ((mode == BP_NORM || (mode == BP_SIRT && a.wslot) || mode == BP_SUM) && a.img.dtype == IMG_F32 && c->err_d &&
-      rows_path(c, kRowsBp, a.v.nz, a.nt, s) && bp_rows_fits(c->rbp_cols, a.nt) &&
+  if ((mode == BP_NORM || (mode == BP_SIRT && a.wslot) || mode == BP_SUM) && c->err_d &&
+      (a.img.dtype == IMG_F32 ? rows_path(c, kRowsBp, a.v.nz, a.nt, s)
+                              : rows_path(c, kRowsBp16, a.v.nz, a.nt, s) ||
+                                    rows_path(c, kRowsBp16Pad, a.v.nz, a.nt, s)) &&
+      bp_rows_fits(c->rbp_cols, a.nt) &&
       scratch_try(c, (void **)&c->rows_d,
                   row_stack_floats(c->nx, c->ny, a.t0 + a.nt, c->rbp_cols) * sizeof(float))) {
     if ((e = rows_acquire(c, s)) != cudaSuccess ||
         (e = launch_blend_rows(a.img, a.geo, a.t0, a.nt, a.oy, c->ny, c->rbp_cols, mode == BP_NORM,
                                c->rows_d, s)) != cudaSuccess ||
-        (e = launch_bp_rows(mode, a, c->rows_d, c->rbp_cols, s)) != cudaSuccess)
+        (e = launch_bp_rows(mode, a, c->rows_d, c->rbp_cols, a.img.dtype != IMG_F32, s)) !=
+            cudaSuccess)
       return e;
     return rows_release(c, s);
   }
@@ -422,7 +435,7 @@ tr_status sirt_rows(tr_ctx *c, const void *proj, int pdtype, const float *ps, fl
                                c->oy, c->nx, c->ny, c->rows_d, c->rbp_cols, s));
   BpArgs b = bp_args(c, vol, 0, c->th, nullptr, 0, c->nt, gamma);
   set_weights(c, &b);
-  TR_CUDA(c, launch_bp_rows(BP_SIRT, b, c->rows_d, c->rbp_cols, s));
+  TR_CUDA(c, launch_bp_rows(BP_SIRT, b, c->rows_d, c->rbp_cols, false, s));
   TR_CUDA(c, rows_release(c, s));
   return TR_OK;
 }

@@ -273,7 +273,9 @@ cudaError_t launch_blend_rows(const ImgView &im, const TiltGeo *geo, int t0, int
 // Back-projection (BP_NORM, BP_SIRT or BP_SUM) from the row stack that
 // launch_blend_rows(margin = cols, norm = mode == BP_NORM) made; cols: the
 // tile's window.
-cudaError_t launch_bp_rows(int mode, const BpArgs &a, const float *rows, int cols, cudaStream_t s);
+// kahan: compensated sums, for stacks that 16 bits held.
+cudaError_t launch_bp_rows(int mode, const BpArgs &a, const float *rows, int cols, bool kahan,
+                           cudaStream_t s);
 // Forward projection added into a row stack of margin `cols`; a.val is not
 // used.
 cudaError_t launch_fp_rows(const FpArgs &a, float *rows, int cols, int nsm, cudaStream_t s);

@@ -81,9 +81,13 @@ __device__ __forceinline__ RowTilt row_tilt(const TiltGeo &g, int xc, int zc, fl
 // Voxel of position i on the snake path over a 4 x 4 patch: i / 4 along the
 // outer axis, forwards and backwards in turn along the inner one.
 __host__ __device__ constexpr int snake_inner(int i) { return (i >> 2) & 1 ? 3 - (i & 3) : i & 3; }
-template <bool XIN>
+// HALVES 1: the same over 4 (x) x 2 (z) voxels, the patch of the compensated
+// back-projection.
+template <bool XIN, int HALVES = 2>
 __host__ __device__ constexpr int snake_voxel(int i) {  // z * 4 + x
-  return XIN ? (i >> 2) * 4 + snake_inner(i) : snake_inner(i) * 4 + (i >> 2);
+  return XIN          ? (i >> 2) * 4 + snake_inner(i)
+         : HALVES == 2 ? snake_inner(i) * 4 + (i >> 2)
+                      : ((i & 1) ^ (i >> 1 & 1)) * 4 + (i >> 1);
 }
 
 // Float offset of column k (>= -margin) of row block yb in a row stack of nyb
@@ -128,12 +132,12 @@ struct __align__(16) PatchPath {
 //   gather: positions 0 and 8 hold the window offset of their lower column, a
 //     crossing position that of the column to load.
 //   splat: a crossing position holds the offset of the column to add to.
-template <bool SPLAT>
+template <bool SPLAT, int HALVES = 2>
 __device__ __forceinline__ void path_records(const RowTilt &tl, int px, int pz, int lane, int pnx,
                                              PatchPath *path) {
-  const int pos = lane & 15, out = pos >> 2, in = snake_inner(pos);
-  const bool xin = tl.flags & 1;
-  const long long U = tl.u0 + (px + (xin ? in : out)) * tl.sx + (pz + (xin ? out : in)) * tl.sz;
+  const int pos = lane & 15, i = pos & (8 * HALVES - 1);  // HALVES 1: the upper 8 repeat
+  const int v = tl.flags & 1 ? snake_voxel<true, HALVES>(i) : snake_voxel<false, HALVES>(i);
+  const long long U = tl.u0 + (px + (v & 3)) * tl.sx + (pz + (v >> 2)) * tl.sz;
   const int k = (int)(U >> 32);
   const float w = fabsf((float)(int)(unsigned)(U >> 1)) * 4.656612873077393e-10f;  // 2^-31
   const int kp = __shfl_up_sync(0xffffffffu, k, 1);
@@ -163,21 +167,23 @@ __device__ __forceinline__ void lds4(f32x2 &a, f32x2 &b, unsigned addr) {
 // One tilt of a patch: win is the lane's window address.  The path is walked in
 // two halves side by side, whose loads overlap.  CHECK: positions outside
 // `valid` get nothing.
-template <bool XIN, bool CHECK>
-__device__ __forceinline__ void gather_patch(f32x2 (&acc)[16][2], unsigned win, const PatchPath *path,
-                                             unsigned mask_ev, unsigned mask_od, unsigned valid) {
-  f32x2 ev[2][2], od[2][2];
-  uint2 r[2][2];  // the records of this step and the next
+template <bool XIN, bool CHECK, int HALVES>
+__device__ __forceinline__ void gather_patch(f32x2 (&acc)[8 * HALVES][2], unsigned win,
+                                             const PatchPath *path, unsigned mask_ev,
+                                             unsigned mask_od, unsigned valid) {
+  f32x2 ev[HALVES][2], od[HALVES][2];
+  uint2 r[2][HALVES];  // the records of this step and the next
   auto fetch = [&](int j) {
-    r[j & 1][0] = *reinterpret_cast<const uint2 *>(path->pos + j);
-    r[j & 1][1] = *reinterpret_cast<const uint2 *>(path->pos + 8 + j);
+#pragma unroll
+    for (int h = 0; h < HALVES; ++h)
+      r[j & 1][h] = *reinterpret_cast<const uint2 *>(path->pos + 8 * h + j);
   };
   fetch(0);
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     if (j + 1 < 8) fetch(j + 1);
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < HALVES; ++h) {
       const int i = 8 * h + j;
       const unsigned at = win + r[j & 1][h].y;
       if (j == 0) {
@@ -195,8 +201,8 @@ __device__ __forceinline__ void gather_patch(f32x2 (&acc)[16][2], unsigned win, 
       }
     }
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int i = 8 * h + j, v = snake_voxel<XIN>(i);
+    for (int h = 0; h < HALVES; ++h) {
+      const int i = 8 * h + j, v = snake_voxel<XIN, HALVES>(i);
       const float wf = __uint_as_float(r[j & 1][h].x);
       const f32x2 w = pack2(wf, wf);
       const f32x2 r0 = fma2(w, sub2(od[h][0], ev[h][0]), ev[h][0]);
@@ -227,7 +233,10 @@ __device__ __forceinline__ void load_quad(const float *p, bool in, bool vec, int
 // Patches of a tile along x and z, a warp each; tiles per SM at 16 warps.
 constexpr int kBpPX = kRowBpX / 4, kBpPZ = kRowBpZ / 4, kBpWarps = kBpPX * kBpPZ;
 constexpr int kBpPerSm = 16 / kBpWarps;
-constexpr int kBpQuads = 4 * kBpPZ * kBpPX;  // float4s of a tile's row, all sections
+// Float4s of a tile's row, all sections: patches have 2 HALVES sections.
+template <int HALVES>
+constexpr int kBpQuads = 2 * HALVES * kBpPZ * kBpPX;
+constexpr int kKahanTilts = 16;  // tilts summed plainly between compensated additions
 constexpr int kLag = 4;  // a stage is refilled kLag tilts after its use
 
 // Back-projection.  Volume tile of 16 (x) x 8 (z) voxels and 128 rows; warp w
@@ -241,12 +250,18 @@ constexpr int kLag = 4;  // a stage is refilled kLag tilts after its use
 // kernel takes 7 with one row per table entry; shared memory 42 %, L2 17 %.
 // 1024 x 1024 x 256 voxels, 61 tilts: 3.83 ms with the row stack's 0.15 ms,
 // from 6.69 ms by the general kernel (4.3e12 from 2.4e12 voxel-tilts/s).
-template <int MODE>
+//
+// KAHAN, for stacks that 16 bits held: 16 x 4 voxels, patches 4 x 2, since the
+// sums of a 4 x 4 patch with totals and corrections take 192 registers.  The
+// same volume: 6.17 ms from 6.90 ms by the general kernel.
+template <int MODE, bool KAHAN>
 __global__ void __launch_bounds__(kBpWarps * 32, kBpPerSm)
     bp_rows_kernel(const BpArgs a, const float *__restrict__ rows, int cols, int stages) {
   extern __shared__ __align__(128) unsigned char dsm[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int xc = blockIdx.x * kRowBpX, zl = blockIdx.y * kRowBpZ, yc = blockIdx.z * kRowTile;
+  constexpr int HALVES = KAHAN ? 1 : 2, VZ = 2 * HALVES, TZ = VZ * kBpPZ;
+  constexpr int Q = kBpQuads<HALVES>;
+  const int xc = blockIdx.x * kRowBpX, zl = blockIdx.y * TZ, yc = blockIdx.z * kRowTile;
   const int nt = a.nt;
   const unsigned win_bytes = (unsigned)cols * kColBytes;
   const unsigned stage_bytes = win_bytes + kBpWarps * (unsigned)sizeof(PatchPath);
@@ -261,7 +276,7 @@ __global__ void __launch_bounds__(kBpWarps * 32, kBpPerSm)
     }
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   for (int i = tid; i < nt; i += blockDim.x)
-    tt[i] = row_tilt(a.geo[a.t0 + i], xc, zl + a.v.zoff, a.ox, a.oz, kRowBpX - 1, kRowBpZ - 1, a.img.nx,
+    tt[i] = row_tilt(a.geo[a.t0 + i], xc, zl + a.v.zoff, a.ox, a.oz, kRowBpX - 1, TZ - 1, a.img.nx,
                      cols);
   __syncthreads();
 
@@ -277,7 +292,7 @@ __global__ void __launch_bounds__(kBpWarps * 32, kBpPerSm)
 #pragma unroll 1
     for (int b = 0; b < kBpWarps / 2; ++b) {
       const int w = 2 * b + (lane >> 4);
-      path_records<false>(tl, w % kBpPX * 4, w / kBpPX * 4, lane, a.img.nx, paths + w);
+      path_records<false, HALVES>(tl, w % kBpPX * 4, w / kBpPX * VZ, lane, a.img.nx, paths + w);
     }
     __syncwarp();
     if (lane == 0) mbar_expect_tx(full + s, win_bytes);  // the stage's one arrival
@@ -286,15 +301,20 @@ __global__ void __launch_bounds__(kBpWarps * 32, kBpPerSm)
 
   // The tile's voxels are read at the end: into L2 meanwhile, one 64-byte
   // segment (a section's 16 x) per row and section.
-  for (int i = tid; i < kRowTile * kRowBpZ; i += kBpWarps * 32) {
-    const int y = yc + i / kRowBpZ, z = zl + i % kRowBpZ;
+  for (int i = tid; i < kRowTile * TZ; i += kBpWarps * 32) {
+    const int y = yc + i / TZ, z = zl + i % TZ;
     if (y < a.v.ny && z < a.v.nz)
       asm volatile("prefetch.global.L2 [%0];" ::"l"(a.v.vol + (size_t)y * a.v.sy +
                                                      (size_t)z * a.v.sz + xc));
   }
-  f32x2 acc[16][2];
+  // KAHAN: kKahanTilts tilts sum into acc, which joins the voxel's total by one
+  // compensated addition (comp: what the total's last addition lost).
+  f32x2 acc[8 * HALVES][2], total[KAHAN ? 8 : 1][2], comp[KAHAN ? 8 : 1][2];
 #pragma unroll
-  for (int v = 0; v < 16; ++v) acc[v][0] = acc[v][1] = 0ull;
+  for (int v = 0; v < 8 * HALVES; ++v) {
+    acc[v][0] = acc[v][1] = 0ull;
+    if (KAHAN) total[v][0] = total[v][1] = comp[v][0] = comp[v][1] = 0ull;
+  }
 
   bool ok = true;
   int s = 0;            // stage of tilt t, and the parity of its use
@@ -320,14 +340,25 @@ __global__ void __launch_bounds__(kBpWarps * 32, kBpPerSm)
     if (m.w & 2) {
       // nothing of the stack in reach
     } else if (MODE == BP_NORM && m.z != 0xffffu) {
-      if (m.w & 1) gather_patch<true, true>(acc, win, path, m.x, m.y, m.z);
-      else gather_patch<false, true>(acc, win, path, m.x, m.y, m.z);
+      if (m.w & 1) gather_patch<true, true, HALVES>(acc, win, path, m.x, m.y, m.z);
+      else gather_patch<false, true, HALVES>(acc, win, path, m.x, m.y, m.z);
     } else {
-      if (m.w & 1) gather_patch<true, false>(acc, win, path, m.x, m.y, m.z);
-      else gather_patch<false, false>(acc, win, path, m.x, m.y, m.z);
+      if (m.w & 1) gather_patch<true, false, HALVES>(acc, win, path, m.x, m.y, m.z);
+      else gather_patch<false, false, HALVES>(acc, win, path, m.x, m.y, m.z);
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(empty + s);
+    if (KAHAN && (t % kKahanTilts == kKahanTilts - 1 || t + 1 == nt)) {
+#pragma unroll
+      for (int v = 0; v < 8 * HALVES; ++v)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const f32x2 y = sub2(acc[v][h], comp[v][h]), u = add2(total[v][h], y);
+          comp[v][h] = sub2(sub2(u, total[v][h]), y);
+          total[v][h] = u;
+          acc[v][h] = 0ull;
+        }
+    }
     if (++s == stages) s = 0, parity ^= 1u;
   }
   if (__syncthreads_or(!ok)) {
@@ -345,33 +376,33 @@ __global__ void __launch_bounds__(kBpWarps * 32, kBpPerSm)
   // Epilogue.  The sums go through shared memory, [row][section][16 x] with
   // the 16-byte pieces of a row exchanged so that neither side meets in a
   // bank, and the volume is read and written by sections' rows of 64 bytes.
-  float4 *sum = reinterpret_cast<float4 *>(dsm);  // [128][kBpQuads]
+  float4 *sum = reinterpret_cast<float4 *>(dsm);  // [128][Q]
   {
-    const int px = warp % kBpPX, pz = warp / kBpPX * 4;
+    const int px = warp % kBpPX, pz = warp / kBpPX * VZ;
 #pragma unroll
     for (int r = 0; r < kLaneRows; ++r)
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
+      for (int k = 0; k < VZ; ++k) {
         float f[4];
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
           float lo, hi;
-          unpack2(acc[k * 4 + x][r >> 1], lo, hi);
+          unpack2(KAHAN ? total[KAHAN ? k * 4 + x : 0][r >> 1] : acc[k * 4 + x][r >> 1], lo, hi);
           f[x] = r & 1 ? hi : lo;
         }
-        sum[(lane * 4 + r) * kBpQuads + (((pz + k) * kBpPX + px) ^ (lane & 7))] =
+        sum[(lane * 4 + r) * Q + (((pz + k) * kBpPX + px) ^ (lane & 7))] =
             make_float4(f[0], f[1], f[2], f[3]);
       }
   }
   __syncthreads();
-  const int quad = lane % kBpQuads;
+  const int quad = lane % Q;
   const int x0 = xc + quad % kBpPX * 4, z = zl + quad / kBpPX;
   const bool inz = z < a.v.nz && x0 < a.v.nx;
   const bool vec = rows_vec(a.v, x0);
   const int gx = (a.v.nx + kTX - 1) / kTX, gy = (a.v.ny + kTY - 1) / kTY;
   constexpr int kBatch = 8;  // rows whose reads are in flight together
-  constexpr int kStep = 32 / kBpQuads;  // rows a warp takes at a time
-  const int row0 = warp * (kRowTile / kBpWarps) + lane / kBpQuads;
+  constexpr int kStep = 32 / Q;  // rows a warp takes at a time
+  const int row0 = warp * (kRowTile / kBpWarps) + lane / Q;
 #pragma unroll 1
   for (int i0 = 0; i0 < kRowTile / kBpWarps / kStep; i0 += kBatch) {
     float old[kBatch][4], scale[kBatch];
@@ -393,7 +424,7 @@ __global__ void __launch_bounds__(kBpWarps * 32, kBpPerSm)
     for (int i = 0; i < kBatch; ++i) {
       const int row = row0 + (i0 + i) * kStep, y = yc + row;
       if (!inz || y >= a.v.ny) continue;
-      const float4 q = sum[row * kBpQuads + (quad ^ ((row >> 2) & 7))];
+      const float4 q = sum[row * Q + (quad ^ ((row >> 2) & 7))];
       const float s[4] = {q.x, q.y, q.z, q.w};
       const float sc = MODE == BP_SIRT ? (scale[i] != 0.f ? a.gamma / scale[i] : 0.f) : a.gamma;
 #pragma unroll
@@ -1000,23 +1031,33 @@ static int fp_rows_slots(int cols, int nt) {
 }
 bool fp_rows_fits(int cols, int nt) { return fp_rows_slots(cols, nt) > 0; }
 
-template <int MODE>
+template <int MODE, bool KAHAN>
 static cudaError_t launch_bp_rows_t(const BpArgs &a, const float *rows, int cols, cudaStream_t s) {
   const int stages = bp_rows_stages(cols, a.nt);
-  const size_t smem = std::max<size_t>(bp_rows_smem(cols, a.nt, stages), kRowTile * kBpQuads * 16);
-  cudaError_t e = cudaFuncSetAttribute(bp_rows_kernel<MODE>,
+  const size_t smem = std::max<size_t>(bp_rows_smem(cols, a.nt, stages),
+                                       kRowTile * kBpQuads<KAHAN ? 1 : 2> * 16);
+  cudaError_t e = cudaFuncSetAttribute(bp_rows_kernel<MODE, KAHAN>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  const dim3 grid((a.v.nx + kRowBpX - 1) / kRowBpX, (a.v.nz + kRowBpZ - 1) / kRowBpZ,
+  const int tz = KAHAN ? kRowBpZ / 2 : kRowBpZ;
+  const dim3 grid((a.v.nx + kRowBpX - 1) / kRowBpX, (a.v.nz + tz - 1) / tz,
                   (a.v.ny + kRowTile - 1) / kRowTile);
-  bp_rows_kernel<MODE><<<grid, kBpWarps * 32, smem, s>>>(a, rows, cols, stages);
+  bp_rows_kernel<MODE, KAHAN><<<grid, kBpWarps * 32, smem, s>>>(a, rows, cols, stages);
   return cudaGetLastError();
 }
 
-cudaError_t launch_bp_rows(int mode, const BpArgs &a, const float *rows, int cols, cudaStream_t s) {
-  if (mode == BP_NORM) return launch_bp_rows_t<BP_NORM>(a, rows, cols, s);
-  if (mode == BP_SIRT) return launch_bp_rows_t<BP_SIRT>(a, rows, cols, s);
-  return launch_bp_rows_t<BP_SUM>(a, rows, cols, s);
+template <bool KAHAN>
+static cudaError_t launch_bp_rows_k(int mode, const BpArgs &a, const float *rows, int cols,
+                                    cudaStream_t s) {
+  if (mode == BP_NORM) return launch_bp_rows_t<BP_NORM, KAHAN>(a, rows, cols, s);
+  if (mode == BP_SIRT) return launch_bp_rows_t<BP_SIRT, KAHAN>(a, rows, cols, s);
+  return launch_bp_rows_t<BP_SUM, KAHAN>(a, rows, cols, s);
+}
+
+cudaError_t launch_bp_rows(int mode, const BpArgs &a, const float *rows, int cols, bool kahan,
+                           cudaStream_t s) {
+  return kahan ? launch_bp_rows_k<true>(mode, a, rows, cols, s)
+               : launch_bp_rows_k<false>(mode, a, rows, cols, s);
 }
 
 cudaError_t launch_fp_rows(const FpArgs &a, float *rows, int cols, int nsm, cudaStream_t s) {

@@ -93,6 +93,24 @@ def test_sirt_and_a_slab_of_sections(engine, restatement, nx, ny, nt, th, layout
     assert float(part.abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("nx,ny,nt,th", [(250, 250, 17, 66), (242, 240, 16, 70),
+                                          (256, 128, 33, 96)])
+def test_compensated_sums_of_16_bit_stacks(engine, restatement, nx, ny, nt, th):
+    """Tilt counts at and beside the groups that are summed plainly.  Plain sums
+    of 16 tilts and one rounding of the total stay within 10 x 2**-24 of sums of
+    like sign; the values here are positive."""
+    R = restatement
+    c8, proj, vol, org = _case(R, nx, ny, nt, th, 0, 60, 0.0)
+    proj, vol = np.abs(proj), np.abs(vol)
+    g = R.geom(nx, ny, nt, th, 0, 0, org)
+    engine.set_problem(nx, ny, nt, th, c8, 0, org)
+    q, scale = engine.quantize(torch.from_numpy(proj).cuda(), torch.float16)
+    exact = (q.float() * scale[:, None, None]).cpu().numpy()
+    v = torch.from_numpy(vol).cuda()
+    engine.backproject_lp(q, scale, v)
+    assert O.rel_l2(v.cpu().numpy(), R.backproject(g, c8, exact, vol, fp64=True)) < 6e-7
+
+
 def test_two_streams_share_a_context(engine, restatement):
     """Back-projections queued on two streams without a synchronisation between
     them each see their own stack."""
