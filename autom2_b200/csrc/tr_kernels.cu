@@ -812,18 +812,24 @@ __device__ __forceinline__ float gather_normalised(const float *__restrict__ img
 }
 
 // The update of a SART sweep: the thread's voxel pairs (FpArgs::simg), read,
-// updated and written back.
-template <bool INSIDE>
+// updated and written back.  tt, sw: the back-projection tile's that holds the
+// pairs, whose Q9.23 coordinates these are, bit by bit, and (SEP) row weights: a
+// voxel at the edge of the image gets its residual or nothing, and a column of
+// voxels there would change with the last bit of its coordinate.
+template <bool SEP, bool INSIDE>
 __device__ __forceinline__ void sart_update_pairs(const FpArgs &a, const TileTilt &tt,
-                                                  const TiltGeo &g, int x, int y, int z0, int lane,
-                                                  int wy, int wz, float (&va)[kFNV],
-                                                  float (&vb)[kFNV]) {
-  const long long A0 = g.A[0], A2 = g.A[2], B0 = g.B[0], B2 = g.B[2];
-  unsigned long long U = (unsigned long long)(tt.U0 + wy * g.A[1] + (long long)(wz * kFNV) * A2 +
-                                              (2 * lane) * A0);
-  unsigned long long V = (unsigned long long)(tt.V0 + wy * g.B[1] + (long long)(wz * kFNV) * B2 +
-                                              (2 * lane) * B0);
+                                                  const SepW &sw, const TiltGeo &g, int x, int y,
+                                                  int z0, int lane, int wy, int wz,
+                                                  float (&va)[kFNV], float (&vb)[kFNV]) {
+  const unsigned dux = q23_step(g.A[0]), du = q23_step(g.A[2]);
+  const unsigned dvx = q23_step(g.B[0]), dv = q23_step(g.B[2]);
+  const unsigned px = (2 * lane) & (kTX - 1);
+  unsigned u = q23((unsigned long long)(tt.U0 + wy * g.A[1] + (long long)(wz * kNV) * g.A[2])) +
+               px * dux;
+  unsigned v = q23((unsigned long long)(tt.V0 + wy * g.B[1] + (long long)(wz * kNV) * g.B[2])) +
+               px * dvx;
   const bool ina = x < a.v.nx && y < a.v.ny, inb = x + 1 < a.v.nx && y < a.v.ny;
+  const bool hit = !SEP || sw.w0 + sw.w1 != 0.f;  // some detector row in reach
   float *p = a.v.vol + (size_t)y * a.v.sy + (size_t)z0 * a.v.sz + x;
   const bool pair = inb && ((a.v.sy | a.v.sz) & 1) == 0 &&
                     (reinterpret_cast<uintptr_t>(a.v.vol) & 7) == 0;
@@ -839,21 +845,19 @@ __device__ __forceinline__ void sart_update_pairs(const FpArgs &a, const TileTil
     va[k] = v.x;
     vb[k] = v.y;
   }
+  auto at = [&](unsigned u, unsigned v) {
+    return gather_normalised<INSIDE>(a.simg, a.pnx, a.pny, tt.kmin + (int)(u >> 23),
+                                     SEP ? sw.y0 : tt.jmin + (int)(v >> 23),
+                                     one_plus_frac23(u) - 1.f,
+                                     SEP ? sw.dy : one_plus_frac23(v) - 1.f);
+  };
 #pragma unroll
   for (int k = 0; k < kFNV; ++k) {
-    const bool inz = z0 + k < a.v.nz;
-    if (inz && ina)
-      va[k] += a.sgamma * gather_normalised<INSIDE>(a.simg, a.pnx, a.pny, tt.kmin + (int)(U >> 32),
-                                                    tt.jmin + (int)(V >> 32),
-                                                    one_plus_frac(U) - 1.f, one_plus_frac(V) - 1.f);
-    const unsigned long long Ub = U + A0, Vb = V + B0;
-    if (inz && inb)
-      vb[k] += a.sgamma * gather_normalised<INSIDE>(a.simg, a.pnx, a.pny, tt.kmin + (int)(Ub >> 32),
-                                                    tt.jmin + (int)(Vb >> 32),
-                                                    one_plus_frac(Ub) - 1.f,
-                                                    one_plus_frac(Vb) - 1.f);
-    U += (unsigned long long)A2;
-    V += (unsigned long long)B2;
+    const bool inz = hit && z0 + k < a.v.nz;
+    if (inz && ina) va[k] += a.sgamma * at(u, v);
+    if (inz && inb) vb[k] += a.sgamma * at(u + dux, v + dvx);
+    u += du;
+    v += dv;
   }
 #pragma unroll
   for (int k = 0; k < kFNV; ++k) {
@@ -889,17 +893,23 @@ __device__ __forceinline__ void fp_tile(const FpArgs &a, int bx, int by, int bz,
 
   float va[kFNV], vb[kFNV];
   if constexpr (SART) {
-    if (tid == 0)
-      tile_setup(*a.sgeo, xc, yc, zc, a.ox, a.oy, a.oz, a.pny, false, kFX - 1, kTY - 1, kFTZ - 1,
-                 tt[0], sw[0]);
+    if (tid < kFX / kTX)  // the back-projection's tiles
+      tile_setup(*a.sgeo, xc + tid * kTX, yc, zc, a.ox, a.oy, a.oz, a.pny, SEP, kTX - 1, kTY - 1,
+                 kFTZ - 1, tt[tid], sw[tid]);
     __syncthreads();
-    const TileTilt t0 = tt[0];
+    const int half = 2 * lane / kTX;
+    const TileTilt t0 = tt[half];
+    const SepW s0 = SEP ? sw[half][wy] : SepW{};
     // the window holds every lower neighbour, its upper one and a margin of one
-    const bool inside = t0.kmin >= 0 && t0.kmin + t0.nq <= a.pnx && t0.jmin >= 0 &&
-                        t0.jmin + t0.nr <= a.pny;
+    const bool inside =
+        t0.kmin >= 0 && t0.kmin + t0.nq <= a.pnx &&
+        (SEP ? s0.y0 >= 0 && s0.y0 + 1 < a.pny : t0.jmin >= 0 && t0.jmin + t0.nr <= a.pny);
     const int x = xc + 2 * lane, y = yc + wy, z0 = zl + wz * kFNV;
-    if (inside) sart_update_pairs<true>(a, t0, *a.sgeo, x, y, z0, lane, wy, wz, va, vb);
-    else sart_update_pairs<false>(a, t0, *a.sgeo, x, y, z0, lane, wy, wz, va, vb);
+    static_assert(kTZ == kFTZ && kNV == kFNV, "the back-projection's z groups");
+    if (__all_sync(0xffffffffu, inside))
+      sart_update_pairs<SEP, true>(a, t0, s0, *a.sgeo, x, y, z0, lane, wy, wz, va, vb);
+    else
+      sart_update_pairs<SEP, false>(a, t0, s0, *a.sgeo, x, y, z0, lane, wy, wz, va, vb);
   } else {
     const int x = xc + 2 * lane, y = yc + wy;
     const bool ina = x < a.v.nx && y < a.v.ny, inb = x + 1 < a.v.nx && y < a.v.ny;

@@ -39,3 +39,21 @@ def test_sart(engine, restatement, nx, ny, nt, th, layout, pitch, rot, shift, it
     engine.sart(torch.from_numpy(proj).cuda(), v, iters, 0.4)
     want = R.sart(R.geom(nx, ny, nt, th, layout, 0, org), c8, proj, vol, iters, 0.4, fp64=True)
     assert O.rel_l2(v.cpu().numpy(), want) < 1e-5
+
+
+def test_sart_whole_pixel_shifts(engine, restatement):
+    """Shifts of whole pixels put voxel rows exactly a pixel above the image,
+    where no tap has a weight: they get nothing.  Tolerance as above."""
+    R = restatement
+    rng = np.random.default_rng(3)
+    nx, ny, nt, th = 66, 12, 3, 20
+    c8 = R.coeffs(np.linspace(-40, 45, nt).astype(np.float32), 0.0, 0.0, 0.0)
+    c8[:, 4] += [-3.0, -1.0, 2.0]
+    proj = rng.normal(size=(nt, ny, nx)).astype(np.float32)
+    vol = np.zeros((ny, th, nx), np.float32)
+    org = T.default_origin(0, nx, ny, th)
+    engine.set_problem(nx, ny, nt, th, c8, 0, org)
+    v = torch.from_numpy(vol.copy()).cuda()
+    engine.sart(torch.from_numpy(proj).cuda(), v, 1, 0.4)
+    want = R.sart(R.geom(nx, ny, nt, th, 0, 0, org), c8, proj, vol, 1, 0.4, fp64=True)
+    assert O.rel_l2(v.cpu().numpy(), want) < 1e-5
