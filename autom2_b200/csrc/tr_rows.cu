@@ -463,19 +463,18 @@ __device__ __forceinline__ void add_col(unsigned addr, f32x2 r0, f32x2 r1) {
   asm volatile("st.shared.v2.u64 [%0], {%1, %2};" ::"r"(addr), "l"(a), "l"(b));
 }
 
-// One tilt of a patch's splat; win: the lane's window address.  Two running
-// sums take the place of EV and OD: all = EV + OD and od = OD, one addition
-// and one fused multiply-add per voxel pair from the record's one weight.  At
-// a crossing one register goes to its column; the column's rows are read a
-// position ahead (successive crossings never add to the same column), and the
-// rest is a real branch (the masks are the same for the whole warp), since
-// predicated instructions would be issued at every position.
+// One tilt of a patch's splat; win: the lane's window address.  Two running sums
+// take the place of EV and OD, a fused multiply-add each per voxel pair.  At a
+// crossing one of them goes to its column and starts again at zero; the column's
+// rows are read a position ahead (successive crossings never add to the same
+// column), and the rest is a real branch (the masks are the same for the whole
+// warp), since predicated instructions would be issued at every position.
 template <bool XIN>
 __device__ __forceinline__ void splat_patch(const f32x2 (&vox)[16][2], unsigned win,
                                             const PatchPath *path) {
   const uint4 m = *reinterpret_cast<const uint4 *>(&path->ev);  // ev, od, last columns
   const unsigned cross = m.x | m.y;
-  f32x2 all0 = 0ull, all1 = 0ull, od0 = 0ull, od1 = 0ull;
+  f32x2 ev0 = 0ull, ev1 = 0ull, od0 = 0ull, od1 = 0ull;
   f32x2 c0 = 0ull, c1 = 0ull;  // rows of the column of the next crossing
   uint2 q[3];
   q[0] = *reinterpret_cast<const uint2 *>(path->pos);
@@ -487,15 +486,13 @@ __device__ __forceinline__ void splat_patch(const f32x2 (&vox)[16][2], unsigned 
       asm volatile(
           "{\n .reg .pred p, q;\n .reg .b32 t, s;\n .reg .b64 c, d;\n"
           " and.b32 t, %7, %9;\n setp.eq.u32 p, t, 0;\n @p bra.uni DONE;\n"
-          " and.b32 s, %8, %9;\n setp.eq.u32 q, s, 0;\n"
-          " sub.rn.f32x2 c, %0, %2;\n sub.rn.f32x2 d, %1, %3;\n @q bra.uni ODD;\n"
-          " add.rn.f32x2 c, %4, c;\n add.rn.f32x2 d, %5, d;\n"
-          " st.shared.v2.u64 [%6], {c, d};\n mov.b64 %0, %2;\n mov.b64 %1, %3;\n bra.uni DONE;\n"
-          "ODD:\n mov.b64 %0, c;\n mov.b64 %1, d;\n add.rn.f32x2 c, %4, %2;\n"
-          " add.rn.f32x2 d, %5, %3;\n st.shared.v2.u64 [%6], {c, d};\n mov.b64 %2, 0;\n"
-          " mov.b64 %3, 0;\n"
+          " and.b32 s, %8, %9;\n setp.eq.u32 q, s, 0;\n @q bra.uni ODD;\n"
+          " add.rn.f32x2 c, %4, %0;\n add.rn.f32x2 d, %5, %1;\n"
+          " st.shared.v2.u64 [%6], {c, d};\n mov.b64 %0, 0;\n mov.b64 %1, 0;\n bra.uni DONE;\n"
+          "ODD:\n add.rn.f32x2 c, %4, %2;\n add.rn.f32x2 d, %5, %3;\n"
+          " st.shared.v2.u64 [%6], {c, d};\n mov.b64 %2, 0;\n mov.b64 %3, 0;\n"
           "DONE:\n}"
-          : "+l"(all0), "+l"(all1), "+l"(od0), "+l"(od1)
+          : "+l"(ev0), "+l"(ev1), "+l"(od0), "+l"(od1)
           : "l"(c0), "l"(c1), "r"(win + q[i % 3].y), "r"(cross), "r"(m.x), "r"(1u << i));
     if (i + 1 < 16)
       asm volatile(
@@ -504,14 +501,14 @@ __device__ __forceinline__ void splat_patch(const f32x2 (&vox)[16][2], unsigned 
           : "+l"(c0), "+l"(c1)
           : "r"(win + q[(i + 1) % 3].y), "r"(cross), "r"(2u << i));
     const int v = snake_voxel<XIN>(i);
-    const float wf = __uint_as_float(q[i % 3].x);
-    const f32x2 w = pack2(wf, wf);
-    all0 = add2(all0, vox[v][0]);
-    all1 = add2(all1, vox[v][1]);
+    const float wf = __uint_as_float(q[i % 3].x), we = 1.f - wf;
+    const f32x2 w = pack2(wf, wf), e = pack2(we, we);
+    ev0 = fma2(e, vox[v][0], ev0);
+    ev1 = fma2(e, vox[v][1], ev1);
     od0 = fma2(w, vox[v][0], od0);
     od1 = fma2(w, vox[v][1], od1);
   }
-  add_col(win + m.z, sub2(all0, od0), sub2(all1, od1));
+  add_col(win + m.z, ev0, ev1);
   add_col(win + m.w, od0, od1);
 }
 
