@@ -512,6 +512,11 @@ __device__ __forceinline__ void splat_patch(const f32x2 (&vox)[16][2], unsigned 
   add_col(win + m.w, od0, od1);
 }
 
+// An empty window: as wide as a row-invariant tile's can be (rfp_cols with steps of
+// at most one).
+constexpr int kZeroCols = kRowFpX + kRowFpZ + 2;
+__device__ __align__(128) float g_zero_window[kZeroCols * kRowTile];
+
 constexpr int kFpPX = kRowFpX / 4, kFpPZ = kRowFpZ / 4, kFpWarps = kFpPX * kFpPZ;
 constexpr int kFpPerSm = 16 / kFpWarps;
 constexpr int kFpQuads = 4 * kFpPZ * kFpPX;
@@ -521,16 +526,20 @@ constexpr int kFpQuads = 4 * kFpPZ * kFpPX;
 // ring of slots and go from warp to warp: warp w adds its patch to a tilt's
 // window once warp w - 1 has, so that no two add to it at a time and the
 // additions need no atomics; the last warp sends the finished window out as one
-// bulk reduction and hands the slot back to the first.  (With all warps in step
-// over eight windows at a time, barriers and the wait for the reductions took a
-// quarter of the time.)
+// bulk reduction, and once that has read it, has a bulk copy clear the slot for the
+// first (whose own stores of zeros took a seventh of the shared-memory wavefronts:
+// 512 x 1024 x 128 voxels, 61 tilts 1613 -> 1568 us).  With all warps in step over
+// eight windows at a time, barriers and the wait for the reductions took a quarter
+// of the time.
 //
-// Bound as the back-projection, with more instructions (7 per voxel and tilt):
-// a column that leaves the path is a read, an addition and a write of its
-// window.  1024 x 1024 x 256 voxels, 61 tilts: 5.74 ms with the row sums'
-// conversion, from 8.12 ms by the general splat, whose 32-bit fixed point this
-// replaces by float sums.  Four warps in the chain and four CTAs per SM: eight
-// and two took 6.07 ms, an 8 x 8 tile 5.90 ms, two warps 5.87 ms.
+// Bound by shared-memory wavefronts (78 % of their peak) and, at 16 warps per SM, by
+// latency (60 % of issue slots); 7.5 instructions per voxel and tilt: a column that
+// leaves the path is a read, an addition and a write of its window.  1024 x 1024 x
+// 256 voxels, 61 tilts: 5.72 ms with the row sums' conversion and the weights, from
+// 8.12 ms by the general splat alone, whose 32-bit fixed point this replaces by
+// float sums.  Four warps in the chain and four CTAs per SM (before the last two
+// changes 5.74 ms without the weights): eight and two took 6.07 ms, an 8 x 8 tile
+// 5.90 ms, two warps 5.87 ms.
 __global__ void __launch_bounds__(kFpWarps * 32, kFpPerSm)
     fp_rows_kernel(const FpArgs a, float *__restrict__ rows, int cols, int slots, int ahead) {
   extern __shared__ __align__(128) unsigned char dsm[];
@@ -541,7 +550,7 @@ __global__ void __launch_bounds__(kFpWarps * 32, kFpPerSm)
   // the windows' room also holds the tile's voxels at first
   RowTilt *tt = reinterpret_cast<RowTilt *>(dsm + max(slots * win_bytes, (unsigned)kRowTile * kFpQuads * 16));
   PatchPath *paths = reinterpret_cast<PatchPath *>(tt + ((nt + 1) & ~1)) + warp * 2;
-  // per slot: warp w has added to it; the last: it may be used again
+  // per slot: warp w has added to it; the last: it holds zeros (again)
   unsigned long long *hand = reinterpret_cast<unsigned long long *>(
       reinterpret_cast<PatchPath *>(tt + ((nt + 1) & ~1)) + kFpWarps * 2);
   for (int i = tid; i < slots * kFpWarps; i += blockDim.x) mbar_init(hand + i, 1);
@@ -609,6 +618,15 @@ __global__ void __launch_bounds__(kFpWarps * 32, kFpPerSm)
 
   float *dst = rows + row_stack_at(a.t0, blockIdx.z, gridDim.z, 0, a.pnx, cols);
   const size_t plane = (size_t)gridDim.z * (a.pnx + 2 * cols) * kRowTile;
+  auto clear = [&](int slot) {  // zeros into a slot, for the first warp's next turn
+    unsigned long long *m = hand + (slot + 1) * kFpWarps - 1;
+    bulk_load(dsm + (size_t)slot * win_bytes, g_zero_window, win_bytes, m);
+    mbar_expect_tx(m, win_bytes);
+  };
+  if (tid == (kFpWarps - 1) * 32) {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    for (int i = 0; i < min(slots, nt); ++i) clear(i);
+  }
   bool ok = true;
   int s = 0;             // slot of tilt t, and the parity of its use
   unsigned parity = 0;
@@ -621,15 +639,7 @@ __global__ void __launch_bounds__(kFpWarps * 32, kFpPerSm)
     }
     unsigned char *win = dsm + (size_t)s * win_bytes;
     unsigned long long *h = hand + s * kFpWarps;
-    if (warp > 0) {
-      ok = mbar_wait_bounded(h + warp - 1, parity, 1ll << 31, a.err);
-    } else {
-      if (t >= slots) ok = mbar_wait_bounded(h + kFpWarps - 1, parity ^ 1u, 1ll << 31, a.err);
-      if (ok)
-        for (unsigned e = lane; e < win_bytes / 16; e += 32)
-          reinterpret_cast<float4 *>(win)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-      __syncwarp();
-    }
+    ok = mbar_wait_bounded(warp > 0 ? h + warp - 1 : h + kFpWarps - 1, parity, 1ll << 31, a.err);
     ok = __all_sync(0xffffffffu, ok);
     if (!ok) break;
     const RowTilt &tl = tt[t];
@@ -647,7 +657,7 @@ __global__ void __launch_bounds__(kFpWarps * 32, kFpPerSm)
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         // the reduction before this one has read its slot
         asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-        if (t > 0) mbar_arrive(hand + (s > 0 ? s : slots) * kFpWarps - 1);
+        if (t > 0 && t - 1 + slots < nt) clear(s > 0 ? s - 1 : slots - 1);
       }
     }
     if (++s == slots) s = 0, parity ^= 1u;
@@ -656,6 +666,10 @@ __global__ void __launch_bounds__(kFpWarps * 32, kFpPerSm)
     atomicExch(a.err, 1);
     atomicExch(a.err + 1, 1);
   }
+  if (!ok && tid == (kFpWarps - 1) * 32)  // a chance for the zeros in flight to land
+    for (int i = 1; i <= slots; ++i)
+      for (unsigned p = 0; p < 2; ++p)
+        mbar_wait_bounded(hand + i * kFpWarps - 1, p, 1ll << 24, nullptr);
   if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
@@ -1026,7 +1040,7 @@ static int fp_rows_slots(int cols, int nt) {
       if (fp_rows_smem(cols, nt, n) <= room) return n;
   return 0;
 }
-bool fp_rows_fits(int cols, int nt) { return fp_rows_slots(cols, nt) > 0; }
+bool fp_rows_fits(int cols, int nt) { return cols <= kZeroCols && fp_rows_slots(cols, nt) > 0; }
 
 template <int MODE, bool KAHAN>
 static cudaError_t launch_bp_rows_t(const BpArgs &a, const float *rows, int cols, cudaStream_t s) {
