@@ -1146,17 +1146,21 @@ tr_status tr_sart(tr_ctx *c, const float *proj, float *vol, int iters, float gam
     return st;
   if ((st = ensure_wt(c, s))) return st;
   const int steps = iters * c->nt;
+  // Sweeps: the deterministic flush has no such form, a single tilt's residual
+  // plane is in use, and two of a wide window's tables would not fit.
+  const bool sweep = !c->deterministic && c->nt > 1 &&
+                     sart_tables(c->sep, c->fw, c->fh) <= kSmemMax / 2;
   for (int i = 0; i < steps; ++i) {
     const int t = i % c->nt;
     float *vt = c->val_d + plane * t;
     // The volume's projection at the first tilt; later ones come with the update
-    // of the tilt before (the deterministic flush has no such form).
-    if (i == 0 || c->deterministic) {
+    // of the tilt before.
+    if (i == 0 || !sweep) {
       TR_CUDA(c, cudaMemsetAsync(vt, 0, plane * sizeof(float), s));
       TR_TRY(run_fp(c, fp_args(c, vol, 0, c->th, c->val_d, t, 1), s));
     }
     TR_CUDA(c, launch_resid(proj + plane * t, vt, c->wt_d + plane * t, plane, c->nsm, s));
-    if (i + 1 < steps && !c->deterministic && c->nt > 1) {
+    if (i + 1 < steps && sweep) {
       const int n = (i + 1) % c->nt;
       TR_CUDA(c, cudaMemsetAsync(c->val_d + plane * n, 0, plane * sizeof(float), s));
       FpArgs f = fp_args(c, vol, 0, c->th, c->val_d, n, 1);
@@ -1164,13 +1168,11 @@ tr_status tr_sart(tr_ctx *c, const float *proj, float *vol, int iters, float gam
       f.simg = vt;
       f.sgeo = c->geo_d + t;
       f.sgamma = gamma;
+      f.sfw = c->fw;
+      f.sfh = c->fh;
       TR_CUDA(c, launch_sart_sweep(c->sep, f, s));
     } else {
       TR_CUDA(c, run_bp(c, BP_NORM, bp_args(c, vol, 0, c->th, c->val_d, t, 1, gamma), s));
-      if (i + 1 < steps && !c->deterministic) {  // a single tilt: its residual plane is in use
-        TR_CUDA(c, cudaMemsetAsync(vt, 0, plane * sizeof(float), s));
-        TR_TRY(run_fp(c, fp_args(c, vol, 0, c->th, c->val_d, t, 1), s));
-      }
     }
   }
   return TR_OK;

@@ -126,6 +126,7 @@ struct FpArgs {
   const float *simg;
   const TiltGeo *sgeo;
   float sgamma;
+  int sfw, sfh;       // the back-projection's window
 };
 
 // Footprint bookkeeping of one tilt for one tile, computed in FP64.
@@ -249,6 +250,10 @@ cudaError_t launch_classify_tiles(const TiltGeo *geo, int nt, const VolView &v, 
 cudaError_t launch_sep_row_weights(const TiltGeo *geo, int nt, int ny, float oy, int pny,
                                    float *wrow, cudaStream_t s);
 cudaError_t launch_fp(bool sep, const FpArgs &a, cudaStream_t s);
+// Shared memory of a sweep's two interpolation tables (windows of fw x fh).
+inline size_t sart_tables(bool sep, int fw, int fh) {
+  return 2 * (size_t)(sep ? kTY : fh) * fw * sizeof(float2);
+}
 // The back-projection update of one tilt and the forward projection of another
 // in one pass over the volume (FpArgs::simg).
 cudaError_t launch_sart_sweep(bool sep, const FpArgs &a, cudaStream_t s);

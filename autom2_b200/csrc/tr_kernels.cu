@@ -790,46 +790,22 @@ struct FpShared {
   int nonzero;
 };
 
-// s/c of the reference's normalised back-projection (BackProject, main-mpi.cpp:
-// 411-450) for a lower neighbour (k, j) and fractions fu, fv: the edge-clamped
-// image's bilinear value where that neighbour lies in [-1, nx-1] x [-1, ny-1],
-// nothing elsewhere.  INSIDE: all four taps are in the image.
-template <bool INSIDE>
-__device__ __forceinline__ float gather_normalised(const float *__restrict__ img, int nx, int ny,
-                                                   int k, int j, float fu, float fv) {
-  float p00, p01, p10, p11;
-  if (INSIDE) {
-    const float *p = img + (size_t)j * nx + k;
-    p00 = __ldg(p), p01 = __ldg(p + 1), p10 = __ldg(p + nx), p11 = __ldg(p + nx + 1);
-  } else {
-    if (k < -1 || k > nx - 1 || j < -1 || j > ny - 1) return 0.f;
-    const int k0 = max(k, 0), k1 = min(k + 1, nx - 1);
-    const float *p = img + (size_t)max(j, 0) * nx, *q = img + (size_t)min(j + 1, ny - 1) * nx;
-    p00 = __ldg(p + k0), p01 = __ldg(p + k1), p10 = __ldg(q + k0), p11 = __ldg(q + k1);
-  }
-  const float r0 = fmaf(fu, p01 - p00, p00), r1 = fmaf(fu, p11 - p10, p10);
-  return fmaf(fv, r1 - r0, r0);
-}
-
 // The update of a SART sweep: the thread's voxel pairs (FpArgs::simg), read,
-// updated and written back.  tt, sw: the back-projection tile's that holds the
-// pairs, whose Q9.23 coordinates these are, bit by bit, and (SEP) row weights: a
+// updated and written back.  The residual comes through the back-projection's
+// interpolation tables (sfh rows of sfw entries at accs, one for each of the
+// back-projection's two tiles that this one covers) at its Q9.23 coordinates: a
 // voxel at the edge of the image gets its residual or nothing, and a column of
 // voxels there would change with the last bit of its coordinate.
-template <bool SEP, bool INSIDE>
-__device__ __forceinline__ void sart_update_pairs(const FpArgs &a, const TileTilt &tt,
-                                                  const SepW &sw, const TiltGeo &g, int x, int y,
-                                                  int z0, int lane, int wy, int wz,
-                                                  float (&va)[kFNV], float (&vb)[kFNV]) {
-  const unsigned dux = q23_step(g.A[0]), du = q23_step(g.A[2]);
-  const unsigned dvx = q23_step(g.B[0]), dv = q23_step(g.B[2]);
-  const unsigned px = (2 * lane) & (kTX - 1);
-  unsigned u = q23((unsigned long long)(tt.U0 + wy * g.A[1] + (long long)(wz * kNV) * g.A[2])) +
-               px * dux;
-  unsigned v = q23((unsigned long long)(tt.V0 + wy * g.B[1] + (long long)(wz * kNV) * g.B[2])) +
-               px * dvx;
+template <bool SEP>
+__device__ __forceinline__ void sart_update(const FpArgs &a, int xc, int yc, int zl, int zc,
+                                            float *accs, TileTilt *tt, SepW (*sw)[kTY],
+                                            float (&va)[kFNV], float (&vb)[kFNV]) {
+  static_assert(kTZ == kFTZ && kNV == kFNV && kFX == 2 * kTX, "the back-projection's tiles");
+  const int tid = threadIdx.x, lane = tid & 31, wy = (tid >> 5) % kTY, wz = (tid >> 5) / kTY;
+  const int x = xc + 2 * lane, y = yc + wy, z0 = zl + wz * kFNV;
+  const TiltGeo &g = *a.sgeo;
+  // the voxels' reads are in flight while the tables are made
   const bool ina = x < a.v.nx && y < a.v.ny, inb = x + 1 < a.v.nx && y < a.v.ny;
-  const bool hit = !SEP || sw.w0 + sw.w1 != 0.f;  // some detector row in reach
   float *p = a.v.vol + (size_t)y * a.v.sy + (size_t)z0 * a.v.sz + x;
   const bool pair = inb && ((a.v.sy | a.v.sz) & 1) == 0 &&
                     (reinterpret_cast<uintptr_t>(a.v.vol) & 7) == 0;
@@ -845,30 +821,71 @@ __device__ __forceinline__ void sart_update_pairs(const FpArgs &a, const TileTil
     va[k] = v.x;
     vb[k] = v.y;
   }
+  if (tid < 2)
+    tile_setup(g, xc + tid * kTX, yc, zc, a.ox, a.oy, a.oz, a.pny, SEP, kTX - 1, kTY - 1, kTZ - 1,
+               tt[tid], sw[tid]);
+  __syncthreads();
+  const int fw = a.sfw, fh = SEP ? kTY : a.sfh, pnx = a.pnx, pny = a.pny;
+  float2 *tbl = reinterpret_cast<float2 *>(accs);
+  EntryWalk w(tid, fh, fw);
+  for (int e = tid; e < 2 * fh * fw; e += kThreads, w.next(fh, fw)) {
+    const TileTilt &t = tt[w.i];
+    if (w.r >= t.nr || w.q >= t.nq) continue;
+    const int x0 = t.kmin + w.q, j = t.jmin + w.r;
+    float b = 0.f, n = 0.f;
+    if (SEP) {
+      const SepW r = sw[w.i][w.r];
+      if (r.w0 + r.w1 != 0.f && x0 >= -1 && x0 <= pnx - 1) {
+        b = sep_at<BP_NORM>(a.simg, 1.f, pnx, pny, r, x0);
+        n = sep_at<BP_NORM>(a.simg, 1.f, pnx, pny, r, x0 + 1);
+      }
+    } else if (x0 >= -1 && x0 <= pnx - 1 && j >= -1 && j <= pny) {
+      b = img_at<BP_NORM>(a.simg, 1.f, pnx, pny, j, x0);
+      n = img_at<BP_NORM>(a.simg, 1.f, pnx, pny, j, x0 + 1);
+    }
+    tbl[e] = make_float2(b - (n - b), n - b);
+  }
+  __syncthreads();
+  const int half = 2 * lane / kTX;
+  const TileTilt &t = tt[half];
+  const unsigned dux = q23_step(g.A[0]), du = q23_step(g.A[2]);
+  const unsigned dvx = q23_step(g.B[0]), dv = q23_step(g.B[2]);
+  const unsigned px = (2 * lane) % kTX;
+  unsigned u = q23((unsigned long long)(t.U0 + wy * g.A[1] + (long long)(wz * kNV) * g.A[2])) +
+               px * dux;
+  unsigned v = q23((unsigned long long)(t.V0 + wy * g.B[1] + (long long)(wz * kNV) * g.B[2])) +
+               px * dvx;
+  const float2 *T = tbl + (half * fh + (SEP ? wy : 0)) * fw;
+  const int jmin = t.jmin, check = t.check_rows;
   auto at = [&](unsigned u, unsigned v) {
-    return gather_normalised<INSIDE>(a.simg, a.pnx, a.pny, tt.kmin + (int)(u >> 23),
-                                     SEP ? sw.y0 : tt.jmin + (int)(v >> 23),
-                                     one_plus_frac23(u) - 1.f,
-                                     SEP ? sw.dy : one_plus_frac23(v) - 1.f);
+    const float f = one_plus_frac23(u);
+    if (SEP) {
+      const float2 e = T[u >> 23];
+      return fmaf(f, e.y, e.x);
+    }
+    const int r = (int)(v >> 23);
+    const float2 *e = T + r * fw + (int)(u >> 23);
+    const float2 e0 = e[0], e1 = e[fw];
+    const float r0 = fmaf(f, e0.y, e0.x), r1 = fmaf(f, e1.y, e1.x);
+    const float s = fmaf(one_plus_frac23(v) - 1.f, r1 - r0, r0);
+    return check && (unsigned)(jmin + r + 1) > (unsigned)pny ? 0.f : s;
   };
 #pragma unroll
   for (int k = 0; k < kFNV; ++k) {
-    const bool inz = hit && z0 + k < a.v.nz;
-    if (inz && ina) va[k] += a.sgamma * at(u, v);
-    if (inz && inb) vb[k] += a.sgamma * at(u + dux, v + dvx);
+    const float ra = at(u, v), rb = at(u + dux, v + dvx);
     u += du;
     v += dv;
-  }
-#pragma unroll
-  for (int k = 0; k < kFNV; ++k) {
     if (z0 + k >= a.v.nz) continue;
     float *q = p + (size_t)k * a.v.sz;
+    if (ina) va[k] += a.sgamma * ra;
+    if (inb) vb[k] += a.sgamma * rb;
     if (pair) *reinterpret_cast<float2 *>(q) = make_float2(va[k], vb[k]);
     else {
       if (ina) q[0] = va[k];
       if (inb) q[1] = vb[k];
     }
   }
+  __syncthreads();  // the tables' room is the windows'
 }
 
 template <bool SEP, bool DET = false, bool SART = false>
@@ -893,23 +910,7 @@ __device__ __forceinline__ void fp_tile(const FpArgs &a, int bx, int by, int bz,
 
   float va[kFNV], vb[kFNV];
   if constexpr (SART) {
-    if (tid < kFX / kTX)  // the back-projection's tiles
-      tile_setup(*a.sgeo, xc + tid * kTX, yc, zc, a.ox, a.oy, a.oz, a.pny, SEP, kTX - 1, kTY - 1,
-                 kFTZ - 1, tt[tid], sw[tid]);
-    __syncthreads();
-    const int half = 2 * lane / kTX;
-    const TileTilt t0 = tt[half];
-    const SepW s0 = SEP ? sw[half][wy] : SepW{};
-    // the window holds every lower neighbour, its upper one and a margin of one
-    const bool inside =
-        t0.kmin >= 0 && t0.kmin + t0.nq <= a.pnx &&
-        (SEP ? s0.y0 >= 0 && s0.y0 + 1 < a.pny : t0.jmin >= 0 && t0.jmin + t0.nr <= a.pny);
-    const int x = xc + 2 * lane, y = yc + wy, z0 = zl + wz * kFNV;
-    static_assert(kTZ == kFTZ && kNV == kFNV, "the back-projection's z groups");
-    if (__all_sync(0xffffffffu, inside))
-      sart_update_pairs<SEP, true>(a, t0, s0, *a.sgeo, x, y, z0, lane, wy, wz, va, vb);
-    else
-      sart_update_pairs<SEP, false>(a, t0, s0, *a.sgeo, x, y, z0, lane, wy, wz, va, vb);
+    sart_update<SEP>(a, xc, yc, zl, zc, accs, tt, sw, va, vb);
   } else {
     const int x = xc + 2 * lane, y = yc + wy;
     const bool ina = x < a.v.nx && y < a.v.ny, inb = x + 1 < a.v.nx && y < a.v.ny;
@@ -1125,9 +1126,9 @@ __device__ __forceinline__ void fp_tile(const FpArgs &a, int bx, int by, int bz,
 
 // SART's step from one tilt to the next in one pass over the volume: read,
 // update from the residual of the tilt before, write, splat for the tilt after.
-// Taps come straight from the residual plane (a few MB, in L2): a table would be
-// used once.  61 tilts of 512 x 512 on 128 sections, per tilt: 133 us from 157
-// (a forward projection and a back-projection, which read the volume twice).
+// 61 tilts of 512 x 512 on 128 sections, per tilt: 93 us, 118 us with the taps
+// from the residual plane in L2, 157 us as a forward projection and a
+// back-projection, which read the volume twice.
 template <bool SEP>
 __global__ void __launch_bounds__(kThreads, 3) sart_sweep_kernel(const FpArgs a) {
   extern __shared__ __align__(16) float accs[];
@@ -1767,7 +1768,8 @@ static cudaError_t launch_sart_t(const FpArgs &a, size_t smem, cudaStream_t s) {
 }
 
 cudaError_t launch_sart_sweep(bool sep, const FpArgs &a, cudaStream_t s) {
-  const size_t smem = (size_t)a.chunk * (sep ? kTY : a.fh) * a.fw * sizeof(float);
+  const size_t win = (size_t)a.chunk * (sep ? kTY : a.fh) * a.fw * sizeof(float),
+               tables = sart_tables(sep, a.sfw, a.sfh), smem = std::max(win, tables);
   return sep ? launch_sart_t<true>(a, smem, s) : launch_sart_t<false>(a, smem, s);
 }
 
