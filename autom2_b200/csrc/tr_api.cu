@@ -1156,13 +1156,18 @@ tr_status tr_sart(tr_ctx *c, const float *proj, float *vol, int iters, float gam
     // The volume's projection at the first tilt; later ones come with the update
     // of the tilt before.
     if (i == 0 || !sweep) {
-      TR_CUDA(c, cudaMemsetAsync(vt, 0, plane * sizeof(float), s));
+      // a sweep's planes are cleared together
+      TR_CUDA(c, cudaMemsetAsync(vt, 0, (sweep ? c->nt : 1) * plane * sizeof(float), s));
       TR_TRY(run_fp(c, fp_args(c, vol, 0, c->th, c->val_d, t, 1), s));
     }
     TR_CUDA(c, launch_resid(proj + plane * t, vt, c->wt_d + plane * t, plane, c->nsm, s));
     if (i + 1 < steps && sweep) {
       const int n = (i + 1) % c->nt;
-      TR_CUDA(c, cudaMemsetAsync(c->val_d + plane * n, 0, plane * sizeof(float), s));
+      // the next iteration's, of which the last tilt's is this step's residual
+      if (n == 0)
+        TR_CUDA(c, cudaMemsetAsync(c->val_d, 0, (c->nt - 1) * plane * sizeof(float), s));
+      else if (n == c->nt - 1 && i >= c->nt)
+        TR_CUDA(c, cudaMemsetAsync(c->val_d + plane * n, 0, plane * sizeof(float), s));
       FpArgs f = fp_args(c, vol, 0, c->th, c->val_d, n, 1);
       f.chunk = 1;
       f.simg = vt;
