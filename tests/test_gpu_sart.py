@@ -57,3 +57,23 @@ def test_sart_whole_pixel_shifts(engine, restatement):
     engine.sart(torch.from_numpy(proj).cuda(), v, 1, 0.4)
     want = R.sart(R.geom(nx, ny, nt, th, 0, 0, org), c8, proj, vol, 1, 0.4, fp64=True)
     assert O.rel_l2(v.cpu().numpy(), want) < 1e-5
+
+
+@pytest.mark.parametrize("scale", [2.2, 2.4])
+def test_sart_wide_windows(engine, restatement, scale):
+    """A rotated, magnified detector: windows whose two tables just fit a sweep's
+    shared memory, and ones that take separate projections.  Tolerance as above."""
+    R = restatement
+    rng = np.random.default_rng(5)
+    nx, ny, nt, th = 70, 40, 3, 34
+    c8 = R.coeffs(np.linspace(-50, 50, nt).astype(np.float32), 0.0, 0.0, 0.0)
+    a, b = c8[:, :4].copy(), c8[:, 4:].copy()
+    c8[:, :4], c8[:, 4:] = (a - b) * np.sqrt(0.5) * scale, (a + b) * np.sqrt(0.5) * scale
+    proj = rng.normal(size=(nt, ny, nx)).astype(np.float32)
+    vol = rng.normal(size=(ny, th, nx)).astype(np.float32)
+    org = T.default_origin(0, nx, ny, th)
+    engine.set_problem(nx, ny, nt, th, c8, 0, org)
+    v = torch.from_numpy(vol.copy()).cuda()
+    engine.sart(torch.from_numpy(proj).cuda(), v, 2, 0.4)
+    want = R.sart(R.geom(nx, ny, nt, th, 0, 0, org), c8, proj, vol, 2, 0.4, fp64=True)
+    assert O.rel_l2(v.cpu().numpy(), want) < 1e-5
