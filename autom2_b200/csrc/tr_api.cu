@@ -414,11 +414,13 @@ tr_status run_weights(tr_ctx *c, int z0, int nz, int t0, int nt, float *wt, cuda
   return run_fp(c, w, s);
 }
 
-// One SIRT iteration over the whole volume with FP32 residuals on the row-
-// invariant path, the residual formed between the row stacks: *done says
-// whether it ran (else nothing was launched).
-tr_status sirt_rows(tr_ctx *c, const void *proj, int pdtype, const float *ps, float *vol,
-                    float gamma, cudaStream_t s, bool *done) {
+// The whole volume's projection on the row-invariant path, left as the row stack
+// that a back-projection reads next: the FP32 residual against proj, or with no
+// proj ADMM's normalised projection, formed between the row stacks.  *done says
+// whether it ran (else nothing was launched); the caller launches the back-projection
+// and then rows_release.
+tr_status rows_project(tr_ctx *c, const void *proj, int pdtype, const float *ps, const float *vol,
+                       cudaStream_t s, bool *done) {
   const size_t sums = row_stack_floats(c->nx, c->ny, c->nt, c->rfp_cols) * sizeof(float);
   *done = !c->deterministic && rows_path(c, kRowsBp, c->th, c->nt, s) &&
           rows_path(c, kRowsFp, c->th, c->nt, s) && bp_rows_fits(c->rbp_cols, c->nt) &&
@@ -433,6 +435,14 @@ tr_status sirt_rows(tr_ctx *c, const void *proj, int pdtype, const float *ps, fl
                             c->nsm, s));
   TR_CUDA(c, launch_resid_rows(c->rowsum_d, c->rfp_cols, proj, pdtype, ps, c->wt_d, c->geo_d, c->nt,
                                c->oy, c->nx, c->ny, c->rows_d, c->rbp_cols, s));
+  return TR_OK;
+}
+
+// One SIRT iteration over the whole volume with FP32 residuals on that path.
+tr_status sirt_rows(tr_ctx *c, const void *proj, int pdtype, const float *ps, float *vol,
+                    float gamma, cudaStream_t s, bool *done) {
+  TR_TRY(rows_project(c, proj, pdtype, ps, vol, s, done));
+  if (!*done) return TR_OK;
   BpArgs b = bp_args(c, vol, 0, c->th, nullptr, 0, c->nt, gamma);
   set_weights(c, &b);
   TR_CUDA(c, launch_bp_rows(BP_SIRT, b, c->rows_d, c->rbp_cols, false, s));
@@ -1419,10 +1429,18 @@ tr_status tr_admm(tr_ctx *c, const float *proj, float *vol, int outer, int cg_it
   // unnormalised gather over all tilts, plus mu x.
   auto apply = [&](const float *x, float *out) -> tr_status {
     TR_CUDA(c, cudaMemsetAsync(out, 0, V * sizeof(float), s));
-    TR_CUDA(c, cudaMemsetAsync(c->val_d, 0, pn * sizeof(float), s));
-    TR_TRY(run_fp(c, fp_args(c, x, 0, c->th, c->val_d, 0, c->nt), s));
-    TR_CUDA(c, admm_normalize(c->val_d, c->wt_d, pn, nsm, s));
-    TR_CUDA(c, run_bp(c, BP_SUM, bp_args(c, out, 0, c->th, c->val_d, 0, c->nt, 1.f), s));
+    const BpArgs b = bp_args(c, out, 0, c->th, c->val_d, 0, c->nt, 1.f);
+    bool done = false;
+    TR_TRY(rows_project(c, nullptr, TR_DTYPE_F32, nullptr, x, s, &done));
+    if (done) {
+      TR_CUDA(c, launch_bp_rows(BP_SUM, b, c->rows_d, c->rbp_cols, false, s));
+      TR_CUDA(c, rows_release(c, s));
+    } else {
+      TR_CUDA(c, cudaMemsetAsync(c->val_d, 0, pn * sizeof(float), s));
+      TR_TRY(run_fp(c, fp_args(c, x, 0, c->th, c->val_d, 0, c->nt), s));
+      TR_CUDA(c, admm_normalize(c->val_d, c->wt_d, pn, nsm, s));
+      TR_CUDA(c, run_bp(c, BP_SUM, b, s));
+    }
     TR_CUDA(c, admm_add_scaled(out, x, mu, V, nsm, s));
     return TR_OK;
   };
