@@ -31,7 +31,7 @@
 //
 // Coordinates, weights and crossings of a path are the same for all lanes, so
 // the lanes compute them side by side -- lane i position i, two tilts at a
-// time -- and leave them in shared memory as one 16-byte record per position,
+// time -- and leave them in shared memory as one 8-byte record per position,
 // which a step reads as a broadcast.
 #include <cuda.h>
 #include <cuda_bf16.h>
