@@ -207,9 +207,15 @@ bool scratch_try(tr_ctx *c, void **p, size_t bytes) {
 }
 
 // Ends the current problem.  Its scratch buffers stay allocated for the next
-// problem to reuse (a new generation: they count as idle until claimed).
+// problems to reuse (a new generation: they count as idle until claimed); those
+// that no problem has claimed for kIdleProblems in a row are given back, so that
+// one large call does not hold its memory for the context's life.  The device is
+// idle here.
+constexpr unsigned kIdleProblems = 3;
 void release_problem(tr_ctx *c) {
   ++c->gen;
+  for (auto &kv : c->slots)
+    if (*kv.first && c->gen - kv.second.gen > kIdleProblems) scratch_free(c, kv.first);
   c->wt_ready = c->wtvol_ready = false;
   c->have_problem = false;
 }

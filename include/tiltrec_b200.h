@@ -94,9 +94,10 @@ tr_status tr_geometry_from_angles(const float *angles_deg, int ntilt,
  * its cudaDeviceReset.  Scratch buffers (reprojections, weights, filter
  * spectra, host-call staging) are kept across tr_set_problem calls and
  * reused when large enough, so a context that reconstructs many series
- * allocates only when a larger one arrives; under a budget, or when the
- * device is short of memory, buffers the current problem has not used are
- * released first.  tr_scratch_bytes reports the budgeted buffers held;
+ * allocates only when a larger one arrives; a buffer that three problems in
+ * a row have not used is freed at the next tr_set_problem, and under a
+ * budget, or when the device is short of memory, buffers the current problem
+ * has not used are released first.  tr_scratch_bytes reports the budgeted buffers held;
  * tr_destroy frees everything. */
 tr_status tr_create(int device, size_t hbm_budget, tr_ctx **out);
 tr_status tr_destroy(tr_ctx *ctx);
