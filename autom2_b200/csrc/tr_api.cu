@@ -317,6 +317,23 @@ cudaError_t rows_acquire(tr_ctx *c, cudaStream_t s) {
 }
 cudaError_t rows_release(tr_ctx *c, cudaStream_t s) { return cudaEventRecord(c->ev_rows, s); }
 
+// The same launch counted from its first tilt, so that a row stack holds its own
+// tilts only.
+BpArgs own_tilts(BpArgs a) {
+  const size_t elem = a.img.dtype == IMG_F32 ? 4 : 2;
+  a.geo += a.t0;
+  a.img.p = (const float *)((const char *)a.img.p + (size_t)a.t0 * a.img.tstride * elem);
+  if (a.img.scale) a.img.scale += a.t0;
+  a.t0 = 0;
+  return a;
+}
+FpArgs own_tilts(FpArgs a) {
+  a.geo += a.t0;
+  a.val += (size_t)a.t0 * a.tstride;
+  a.t0 = 0;
+  return a;
+}
+
 // Back-projection launch: clears the launch-wide abort word first.
 cudaError_t run_bp(tr_ctx *c, int mode, const BpArgs &a, cudaStream_t s) {
   cudaError_t e;
@@ -327,11 +344,12 @@ cudaError_t run_bp(tr_ctx *c, int mode, const BpArgs &a, cudaStream_t s) {
                                     rows_path(c, kRowsBp16Pad, a.v.nz, a.nt, s)) &&
       bp_rows_fits(c->rbp_cols, a.nt) &&
       scratch_try(c, (void **)&c->rows_d,
-                  row_stack_floats(c->nx, c->ny, a.t0 + a.nt, c->rbp_cols) * sizeof(float))) {
+                  row_stack_floats(c->nx, c->ny, a.nt, c->rbp_cols) * sizeof(float))) {
+    const BpArgs b = own_tilts(a);
     if ((e = rows_acquire(c, s)) != cudaSuccess ||
-        (e = launch_blend_rows(a.img, a.geo, a.t0, a.nt, a.oy, c->ny, c->rbp_cols, mode == BP_NORM,
+        (e = launch_blend_rows(b.img, b.geo, 0, b.nt, b.oy, c->ny, c->rbp_cols, mode == BP_NORM,
                                c->rows_d, s)) != cudaSuccess ||
-        (e = launch_bp_rows(mode, a, c->rows_d, c->rbp_cols, a.img.dtype != IMG_F32, s)) !=
+        (e = launch_bp_rows(mode, b, c->rows_d, c->rbp_cols, b.img.dtype != IMG_F32, s)) !=
             cudaSuccess)
       return e;
     return rows_release(c, s);
@@ -378,16 +396,16 @@ FpArgs fp_args(const tr_ctx *c, const float *vol, int z0, int nz, float *val,
 // tr_set_deterministic the int64 one (sums cleared first, converted after).
 tr_status run_fp(tr_ctx *c, const FpArgs &a, cudaStream_t s) {
   if (!c->deterministic) {
-    const size_t rb =
-        row_stack_floats(c->nx, c->ny, a.t0 + a.nt, c->rfp_cols) * sizeof(float);
+    const size_t rb = row_stack_floats(c->nx, c->ny, a.nt, c->rfp_cols) * sizeof(float);
     if (rows_path(c, kRowsFp, a.v.nz, a.nt, s) && fp_rows_fits(c->rfp_cols, a.nt) &&
         scratch_try(c, (void **)&c->rowsum_d, rb)) {
+      const FpArgs f = own_tilts(a);
       TR_CUDA(c, rows_acquire(c, s));
       TR_CUDA(c, cudaMemsetAsync(c->err_d, 0, sizeof(int), s));
       TR_CUDA(c, cudaMemsetAsync(c->rowsum_d, 0, rb, s));
-      TR_CUDA(c, launch_fp_rows(a, c->rowsum_d, c->rfp_cols, c->nsm, s));
-      TR_CUDA(c, launch_unblend_rows(c->rowsum_d, a.geo, a.t0, a.nt, a.oy, c->ny, c->rfp_cols,
-                                     a.val, a.tstride, c->nx, c->ny, s));
+      TR_CUDA(c, launch_fp_rows(f, c->rowsum_d, c->rfp_cols, c->nsm, s));
+      TR_CUDA(c, launch_unblend_rows(c->rowsum_d, f.geo, 0, f.nt, f.oy, c->ny, c->rfp_cols, f.val,
+                                     f.tstride, c->nx, c->ny, s));
       TR_CUDA(c, rows_release(c, s));
       return TR_OK;
     }

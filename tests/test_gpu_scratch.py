@@ -3,6 +3,7 @@ import numpy as np
 import pytest
 import torch
 
+import oracle as O
 from autom2_b200 import tiltrec as T
 
 pytestmark = pytest.mark.gpu
@@ -35,3 +36,28 @@ def test_scratch_that_no_problem_claims_is_given_back():
         assert e.scratch_bytes > admm
     finally:
         e.close()
+
+
+def test_a_row_stack_holds_the_launch_s_tilts_only():
+    """SART back-projects single tilts of a row-invariant geometry: beside its
+    stacks (and the int64 sums of the deterministic mode) a context holds one
+    tilt's row stack at most, not one that grows to the whole series'.  Both modes
+    agree to the parity bar of the FP32 kernels, relative L2 1e-5."""
+    nx, ny, nt, th = 1024, 512, 6, 64
+    p = torch.randn((nt, ny, nx), device="cuda")
+    got = []
+    for deterministic in (False, True):
+        e = T.Engine(0)
+        try:
+            e.set_problem(nx, ny, nt, th, _tilts(nt))
+            e.set_deterministic(deterministic)
+            v = torch.zeros((ny, th, nx), device="cuda")
+            e.sart(p, v, 1, 0.3)
+            torch.cuda.synchronize()
+            stacks = nt * ny * nx * 4 * (4 if deterministic else 2)
+            tilt = ny * (nx + 2 * 64) * 4  # windows are less than 64 columns wide
+            assert e.scratch_bytes <= stacks + tilt + 4096
+            got.append(v)
+        finally:
+            e.close()
+    assert O.rel_l2(got[0].cpu().numpy(), got[1].cpu().numpy()) < 1e-5
