@@ -193,8 +193,15 @@ bool scratch_try(tr_ctx *c, void **p, size_t bytes) {
   sl.optional = true;
   if (!*p || sl.cap < bytes) {
     if (c->budget && c->scratch - (*p ? sl.cap : 0) + bytes > c->budget) return false;
+    // The calls that come here allocated nothing otherwise, so they may run on one
+    // stream while another stream of the process is being captured, which an
+    // allocation in the thread's default mode would invalidate.
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
     if (*p) scratch_free(c, p);
-    if (cudaMalloc(p, bytes) != cudaSuccess) {
+    const cudaError_t e = cudaMalloc(p, bytes);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) {
       cudaGetLastError();
       *p = nullptr;
       return false;

@@ -61,3 +61,33 @@ def test_a_row_stack_holds_the_launch_s_tilts_only():
         finally:
             e.close()
     assert O.rel_l2(got[0].cpu().numpy(), got[1].cpu().numpy()) < 1e-5
+
+
+def test_a_projection_beside_a_capture():
+    """Projections on a stream of their own, on a context that has no scratch yet,
+    leave the capture of another stream as it is."""
+    nx, ny, nt, th = 512, 256, 41, 64
+    p = torch.randn((nt, ny, nx), device="cuda")
+    v = torch.zeros((ny, th, nx), device="cuda")
+    val = torch.zeros_like(p)
+    x = torch.zeros(8, device="cuda")
+    side = torch.cuda.Stream()
+    e = T.Engine(0)
+    try:
+        e.set_problem(nx, ny, nt, th, _tilts(nt))
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            x += 1
+            with torch.cuda.stream(side):
+                e.backproject(p, v)
+                e.forward_project(v, val)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert e.scratch_bytes > 0  # the row stacks
+        assert float(x.min()) == float(x.max()) == 1.0
+        again = torch.zeros_like(v)
+        e.backproject(p, again)
+        assert torch.equal(v, again)
+    finally:
+        e.close()
