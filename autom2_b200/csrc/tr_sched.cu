@@ -235,22 +235,36 @@ size_t job_bytes(const tr_sched *S, const Job &j) {
 // what finished jobs gave back (the default pool unmaps it at the next
 // synchronisation, and mapping a few hundred MB again takes milliseconds: four
 // series of 512 x 512, WBP and two iterations 10.1 to 25.9 -> 9.2 ms) until the
-// scheduler has been idle for kPoolIdle seconds.
+// scheduler has been idle for kPoolIdle seconds.  What it keeps and what jobs hold
+// stay within the scheduler's budget together (fit_pool).
 constexpr unsigned long long kPoolKeep = 4ull << 30;
 constexpr double kPoolIdle = 1.0;
-cudaMemPool_t make_pool(int device) {
+cudaMemPool_t make_pool(int device, size_t budget) {
   cudaMemPoolProps props{};
   props.allocType = cudaMemAllocationTypePinned;
   props.location.type = cudaMemLocationTypeDevice;
   props.location.id = device;
   cudaMemPool_t pool = nullptr;
-  unsigned long long keep = kPoolKeep;
+  unsigned long long keep = budget ? std::min<unsigned long long>(kPoolKeep, budget) : kPoolKeep;
   if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;  // the device's default pool then
   }
   cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
   return pool;
+}
+// Room for `bytes` more in the pool under the budget: a job whose buffers do not
+// fit what the pool kept reserves new memory beside it, so what would not fit the
+// budget together is given back first.
+tr_status fit_pool(tr_sched *S, size_t bytes) {
+  unsigned long long held = 0;
+  if (!S->pool || !S->budget ||
+      cudaMemPoolGetAttribute(S->pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
+      held + bytes <= S->budget)
+    return TR_OK;
+  SCHED_CUDA(S, cudaStreamSynchronize(S->back));  // finished jobs' frees
+  SCHED_CUDA(S, cudaMemPoolTrimTo(S->pool, S->budget > bytes ? S->budget - bytes : 0));
+  return TR_OK;
 }
 template <typename T>
 cudaError_t alloc(const tr_sched *S, T **p, size_t bytes, cudaStream_t s) {
@@ -663,7 +677,8 @@ tr_status progress(tr_sched *S, bool *busy) {
     S->peak = std::max(S->peak, S->used);
     S->active.push_back(*pick);
     S->queue.erase(pick);
-    tr_status st = admit(S, j);
+    tr_status st = fit_pool(S, j.bytes);
+    if (!st) st = admit(S, j);
     if (st) return st;
     *busy = true;
   }
@@ -735,6 +750,7 @@ void worker(tr_sched *S) {
     }
     if (S->pool && S->pool_since > 0 && S->active.empty() && S->queue.empty() &&
         now_s() - S->pool_since > kPoolIdle) {
+      cudaStreamSynchronize(S->back);  // until then the jobs' frees count as outstanding
       cudaMemPoolTrimTo(S->pool, 0);
       S->pool_since = 0;
     }
@@ -790,7 +806,7 @@ tr_status tr_sched_create(int device, size_t hbm_budget, int proj_dtype, int res
     memset(S->tab_h[b], 0, sizeof(BatchTable));
     if (cudaMemset(S->tab_d[b], 0, sizeof(BatchTable)) != cudaSuccess) return TR_ERR_CUDA;
   }
-  S->pool = make_pool(device);
+  S->pool = make_pool(device, hbm_budget);
   if (configure(S.get(), S->smem_bp, 0)) return S->fatal;
   if (cudaStreamSynchronize(S->s) != cudaSuccess) return TR_ERR_CUDA;
   tr_sched *p = S.release();

@@ -364,7 +364,10 @@ typedef struct {
 
 /* proj_dtype: storage of the stack between steps (TR_DTYPE_F32/F16/BF16,
  * 16-bit with per-tilt power-of-two scales); resid_dtype: SIRT residual
- * storage (FP16 in the stack's scales). */
+ * storage (FP16 in the stack's scales).  Finished jobs' memory is kept for the
+ * next ones, up to 4 GB and within hbm_budget together with what admitted jobs
+ * hold, until the scheduler has been idle for a second; other allocators of the
+ * process do not have it until then. */
 tr_status tr_sched_create(int device, size_t hbm_budget, int proj_dtype,
                           int resid_dtype, tr_sched **out);
 tr_status tr_sched_submit(tr_sched *s, const tr_job *job, unsigned long long *id);
