@@ -345,7 +345,10 @@ FpArgs own_tilts(FpArgs a) {
 cudaError_t run_bp(tr_ctx *c, int mode, const BpArgs &a, cudaStream_t s) {
   cudaError_t e;
   if (c->err_d && (e = cudaMemsetAsync(c->err_d, 0, sizeof(int), s)) != cudaSuccess) return e;
-  if ((mode == BP_NORM || (mode == BP_SIRT && a.wslot) || mode == BP_SUM) && c->err_d &&
+  // The deterministic mode takes the general kernel always: which one runs here
+  // depends on the room for a row stack, and their sums round differently.
+  if (!c->deterministic && (mode == BP_NORM || (mode == BP_SIRT && a.wslot) || mode == BP_SUM) &&
+      c->err_d &&
       (a.img.dtype == IMG_F32 ? rows_path(c, kRowsBp, a.v.nz, a.nt, s)
                               : rows_path(c, kRowsBp16, a.v.nz, a.nt, s) ||
                                     rows_path(c, kRowsBp16Pad, a.v.nz, a.nt, s)) &&

@@ -283,10 +283,13 @@ tr_status tr_sirt_zslabs(tr_ctx *ctx, const void *proj_dev, int proj_dtype,
  * rounded from the same float value the default flush adds), and the sums are
  * converted and added into the output afterwards.  Integer addition is
  * associative, so tr_forward_project and every SIRT / SART / ADMM / z-slab
- * call of the context give bitwise-identical results run to run (the
- * back-projection is deterministic in both modes).  Costs a reduction over
- * the volume, int64 sums of twice the stack's bytes and a conversion pass per
- * forward projection.  Scheduler and tr_sirt_static calls are not affected. */
+ * call of the context give bitwise-identical results run to run.  (A
+ * back-projection repeats its sums exactly in both modes, but with the mode off
+ * the kernel it runs, and with it the rounding, can depend on the scratch
+ * memory there is room for; the deterministic mode needs none for it.)  Costs
+ * a reduction over the volume, int64 sums of twice the stack's bytes and a
+ * conversion pass per forward projection.  Scheduler and tr_sirt_static calls
+ * are not affected. */
 tr_status tr_set_deterministic(tr_ctx *ctx, int on);
 
 /* SIRT over z-slabs from host buffers, the volume staying in host memory

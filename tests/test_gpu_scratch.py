@@ -91,3 +91,52 @@ def test_a_projection_beside_a_capture():
         assert torch.equal(v, again)
     finally:
         e.close()
+
+
+def test_deterministic_results_do_not_depend_on_the_scratch():
+    """The same back-projection, with room for a row stack and with none."""
+    nx, ny, nt, th = 512, 256, 41, 64
+    p = torch.randn((nt, ny, nx), device="cuda")
+    got = []
+    for budget in (0, 1):
+        e = T.Engine(0, hbm_budget=budget)
+        try:
+            e.set_problem(nx, ny, nt, th, _tilts(nt))
+            e.set_deterministic(True)
+            v = torch.zeros((ny, th, nx), device="cuda")
+            e.backproject(p, v)
+            got.append(v)
+        finally:
+            e.close()
+    assert torch.equal(*got)
+
+
+@pytest.mark.parametrize("room", [0, 1, 2])
+def test_sirt_with_room_for_some_of_the_row_stacks(room):
+    """Budgets that hold SIRT's own scratch and none, one or both of the row stacks
+    (the projection's and the back-projection's): the same volume, to the parity bar
+    of the FP32 kernels, and a budget that is kept."""
+    nx, ny, nt, th = 512, 256, 41, 64
+    p = torch.randn((nt, ny, nx), device="cuda")
+    stack = nt * ny * nx * 4
+    want = torch.zeros((ny, th, nx), device="cuda")
+    e = T.Engine(0)
+    try:
+        e.set_problem(nx, ny, nt, th, _tilts(nt))
+        e.set_deterministic(True)
+        e.sirt(p, want, 2, 0.5)
+        # without the int64 sums and the largest magnitude of the deterministic mode
+        need = e.scratch_bytes - 2 * stack - 4
+    finally:
+        e.close()
+    e = T.Engine(0, hbm_budget=need + room * (stack * 5 // 4) + 4096)
+    try:
+        e.set_problem(nx, ny, nt, th, _tilts(nt))
+        v = torch.zeros_like(want)
+        e.sirt(p, v, 2, 0.5)
+        torch.cuda.synchronize()
+        assert e.scratch_bytes <= need + room * (stack * 5 // 4) + 4096
+        assert e.scratch_bytes >= need + room * stack
+        assert O.rel_l2(v.cpu().numpy(), want.cpu().numpy()) < 1e-5
+    finally:
+        e.close()
