@@ -522,7 +522,10 @@ tr_status load_geometry(tr_ctx *c, const double *coeff8, cudaStream_t s) {
   std::vector<TiltGeo> g(nt);
   GeomInfo gi;
   int bad = -1;
-  switch (derive_geometry(coeff8, nt, c->nx, c->ny, c->th, kSmemMax, g.data(), &gi, &bad)) {
+  int gs = derive_geometry(coeff8, nt, c->nx, c->ny, c->th, kSmemMax, g.data(), &gi, &bad);
+  if (gs == GEOM_OK)
+    gs = check_origin(coeff8, nt, c->nx, c->ny, c->th, c->ox, c->oy, c->oz, &gi, &bad);
+  switch (gs) {
     case GEOM_OK: break;
     case GEOM_NONFINITE: return fail(c, TR_ERR_ARG, "non-finite coefficient at tilt %d", bad);
     case GEOM_MAGNITUDE:
@@ -981,11 +984,11 @@ tr_status tr_set_problem(tr_ctx *c, int nx, int ny, int nt, int th, int layout,
     TR_CUDA(c, cudaMalloc(&c->geo_d, sizeof(TiltGeo) * nt));
     c->geo_cap = nt;
   }
-  TR_TRY(load_geometry(c, coeff8, nullptr));
-  c->layout = layout;
   c->ox = ox;
   c->oy = oy;
   c->oz = oz;
+  TR_TRY(load_geometry(c, coeff8, nullptr));
+  c->layout = layout;
   c->have_problem = true;
   return TR_OK;
 }

@@ -146,6 +146,46 @@ inline int derive_geometry(const double *coeff8, int nt, int nx, int ny, int th,
   return GEOM_OK;
 }
 
+// Largest origin coordinate of the row-invariant kernels and the product weights.
+// They take a voxel row's detector row as the row plus floor(b0), give or take
+// one, for the size of their tiles in shared memory; it is formed from the float
+// difference y - oy, which is off by at most 2^-5 px here (y is below 2^18) and by
+// whole pixels once an origin is above 2^24.
+constexpr float kRowsOrigin = 262144.f;
+
+// The origin's part of the checks, after derive_geometry: GEOM_RANGE when a voxel's
+// detector coordinate, formed from float offsets as the kernels form it, is beyond
+// the int range of the window origins or not a number, which every tile's window
+// bookkeeping relies on.  Takes the row-invariant forms from *info where their
+// tiles do not cover the origin's rounding.
+inline int check_origin(const double *coeff8, int nt, int nx, int ny, int th, float ox, float oy,
+                        float oz, GeomInfo *info, int *bad_tilt) {
+  const float o[3] = {ox, oy, oz};
+  const int n[3] = {nx, ny, th};
+  double lo[3], hi[3];
+  for (int i = 0; i < 3; ++i) {
+    lo[i] = (double)(0.f - o[i]);
+    hi[i] = (double)((float)(n[i] - 1) - o[i]);
+    if (!(std::fabs(o[i]) <= kRowsOrigin)) info->rows = info->product_weights = false;
+  }
+  for (int t = 0; t < nt; ++t) {
+    const double *k = coeff8 + 8 * (size_t)t;
+    for (int d = 0; d < 2; ++d) {  // column, row
+      double least = k[4 * d] + (double)o[d], most = least;
+      for (int i = 0; i < 3; ++i) {
+        const double p = k[4 * d + 1 + i] * lo[i], q = k[4 * d + 1 + i] * hi[i];
+        least += std::min(p, q);
+        most += std::max(p, q);
+      }
+      if (!(least >= -1.0e9 && most <= 1.0e9)) {
+        *bad_tilt = t;
+        return GEOM_RANGE;
+      }
+    }
+  }
+  return GEOM_OK;
+}
+
 // Tilts staged per chunk when one tilt's window takes `entry` bytes of a
 // `budget`-byte table.
 inline int chunk_for(size_t budget, size_t entry) {

@@ -341,6 +341,8 @@ tr_status admit(tr_sched *S, Job &j) {
   int bad = -1;
   derive_geometry(j.coeff.data(), nt, j.d.nx, j.d.ny, j.d.thickness, kSchedSmemMax, g.data(),
                   &j.gi, &bad);
+  check_origin(j.coeff.data(), nt, j.d.nx, j.d.ny, j.d.thickness, j.d.ox, j.d.oy, j.d.oz, &j.gi,
+               &bad);
   SCHED_CUDA(S, cudaMemcpyAsync(j.geo, g.data(), sizeof(TiltGeo) * nt, cudaMemcpyHostToDevice,
                                 ps));
   // FP32 projections into val (upload or device copy), then the stored stack.
@@ -831,8 +833,11 @@ tr_status tr_sched_submit(tr_sched *S, const tr_job *job, unsigned long long *id
   j->iters_left = d.sirt_iters;
   std::vector<TiltGeo> g(d.ntilt);
   int bad = -1;
-  const int gs = derive_geometry(j->coeff.data(), d.ntilt, d.nx, d.ny, d.thickness,
-                                 kSchedSmemMax, g.data(), &j->gi, &bad);
+  int gs = derive_geometry(j->coeff.data(), d.ntilt, d.nx, d.ny, d.thickness,
+                           kSchedSmemMax, g.data(), &j->gi, &bad);
+  if (gs == GEOM_OK)
+    gs = check_origin(j->coeff.data(), d.ntilt, d.nx, d.ny, d.thickness, d.ox, d.oy, d.oz, &j->gi,
+                      &bad);
   if (gs == GEOM_NONFINITE) return TR_ERR_ARG;
   if (gs != GEOM_OK) return TR_ERR_UNSUPPORTED;
   std::lock_guard<std::mutex> lk(S->mu);

@@ -82,11 +82,12 @@ struct StaticGeom {
 // Fixed-point steps and tile windows for the coefficients, as the context
 // path derives them; returns the GeomStatus (GEOM_OK when the kernels can
 // stage the geometry).
-int derive(const double *coeff8, int nt, int nx, int ny, int th, TiltGeo *g,
-           StaticGeom *out) {
+int derive(const double *coeff8, int nt, int nx, int ny, int th, float ox, float oy, float oz,
+           TiltGeo *g, StaticGeom *out) {
   GeomInfo gi;
   int bad = -1;
-  const int gs = derive_geometry(coeff8, nt, nx, ny, th, kStaticSmemMax, g, &gi, &bad);
+  int gs = derive_geometry(coeff8, nt, nx, ny, th, kStaticSmemMax, g, &gi, &bad);
+  if (gs == GEOM_OK) gs = check_origin(coeff8, nt, nx, ny, th, ox, oy, oz, &gi, &bad);
   if (gs != GEOM_OK) return gs;
   out->fw = gi.fw;
   out->fh = gi.fh;
@@ -126,7 +127,7 @@ tr_status run(int device, int nx, int ny, int nt, int th, int layout,
 
   TiltGeo g[kStaticMaxTilts];
   StaticGeom sg;
-  const int gs = derive(coeff8, nt, nx, ny, th, g, &sg);
+  const int gs = derive(coeff8, nt, nx, ny, th, ox, oy, oz, g, &sg);
   if (gs == GEOM_NONFINITE) return TR_ERR_ARG;  // as tr_set_problem
   if (gs != GEOM_OK) return TR_ERR_UNSUPPORTED;
 

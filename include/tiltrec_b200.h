@@ -107,7 +107,9 @@ size_t tr_scratch_bytes(const tr_ctx *ctx);
 /* Problem geometry: projection stack nx*ny*ntilt, volume thickness, layout,
  * coefficients (ntilt*8 doubles) and the float origin the reference uses
  * (TiltRec-mpi: (nx/2, th/2, th/2), main-mpi.cpp:743-745;
- *  TiltRecZ:     (nx/2, ny/2, th/2), main-mpiz.cpp:1078-1080). */
+ *  TiltRecZ:     (nx/2, ny/2, th/2), main-mpiz.cpp:1078-1080).
+ * TR_ERR_UNSUPPORTED when a voxel would project beyond +-1e9 pixels (or an
+ * origin is not a number). */
 tr_status tr_set_problem(tr_ctx *ctx, int nx, int ny, int ntilt,
                          int thickness, int layout, const double *coeff8,
                          float ox, float oy, float oz);
