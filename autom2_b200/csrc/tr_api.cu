@@ -407,7 +407,7 @@ FpArgs fp_args(const tr_ctx *c, const float *vol, int z0, int nz, float *val,
 tr_status run_fp(tr_ctx *c, const FpArgs &a, cudaStream_t s) {
   if (!c->deterministic) {
     const size_t rb = row_stack_floats(c->nx, c->ny, a.nt, c->rfp_cols) * sizeof(float);
-    if (rows_path(c, kRowsFp, a.v.nz, a.nt, s) && fp_rows_fits(c->rfp_cols, a.nt) &&
+    if (rows_path(c, kRowsFp, a.v.nz, a.nt, s) && fp_rows_fits(c->rfp_cols) &&
         scratch_try(c, (void **)&c->rowsum_d, rb)) {
       const FpArgs f = own_tilts(a);
       TR_CUDA(c, rows_acquire(c, s));
@@ -458,7 +458,7 @@ tr_status rows_project(tr_ctx *c, const void *proj, int pdtype, const float *ps,
   const size_t sums = row_stack_floats(c->nx, c->ny, c->nt, c->rfp_cols) * sizeof(float);
   *done = !c->deterministic && rows_path(c, kRowsBp, c->th, c->nt, s) &&
           rows_path(c, kRowsFp, c->th, c->nt, s) && bp_rows_fits(c->rbp_cols, c->nt) &&
-          fp_rows_fits(c->rfp_cols, c->nt) && scratch_try(c, (void **)&c->rowsum_d, sums) &&
+          fp_rows_fits(c->rfp_cols) && scratch_try(c, (void **)&c->rowsum_d, sums) &&
           scratch_try(c, (void **)&c->rows_d,
                       row_stack_floats(c->nx, c->ny, c->nt, c->rbp_cols) * sizeof(float));
   if (!*done) return TR_OK;

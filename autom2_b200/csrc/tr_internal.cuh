@@ -269,7 +269,7 @@ inline size_t row_stack_floats(int nx, int ny, int nt, int margin) {
   return (size_t)nt * ((ny + kRowTile - 1) / kRowTile) * kRowTile * (nx + 2 * (size_t)margin);
 }
 bool bp_rows_fits(int cols, int nt);
-bool fp_rows_fits(int cols, int nt);
+bool fp_rows_fits(int cols);
 // Image stack -> voxel-row stack of tilts [t0, t0 + nt): norm, columns -1..nx of
 // the edge-clamped image normalised by the rows' in-image weight; else columns
 // 0..nx-1 of the in-image rows.

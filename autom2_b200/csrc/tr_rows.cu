@@ -1039,13 +1039,29 @@ static size_t fp_rows_smem(int cols, int nt, int slots) {
          slots * kFpWarps * sizeof(unsigned long long);
 }
 // Slots: one in each warp's hands, one being sent out, and some to spare.
-static int fp_rows_slots(int cols, int nt) {
-  for (size_t room : {kRowSmem / kFpPerSm, kRowSmem})
-    for (int n = kFpWarps + 4; n > kFpWarps; --n)
-      if (fp_rows_smem(cols, nt, n) <= room) return n;
+static int fp_rows_slots(int cols, int nt, size_t room) {
+  for (int n = kFpWarps + 4; n > kFpWarps; --n)
+    if (fp_rows_smem(cols, nt, n) <= room) return n;
   return 0;
 }
-bool fp_rows_fits(int cols, int nt) { return cols <= kZeroCols && fp_rows_slots(cols, nt) > 0; }
+// CTAs per SM, and the most tilts of a launch whose bookkeeping leaves the SM room
+// for them: kFpPerSm for the windows of rotations (20 columns at most), half of it
+// for sheared ones.  (512 x 512 x 64 voxels, windows of 20 columns: 150 tilts 1.10
+// ms; 160 tilts in one launch of two CTAs per SM 1.46 ms, as two launches 1.21 ms.)
+struct FpResident {
+  int per_sm, tilts;
+  size_t room;
+};
+static FpResident fp_rows_resident(int cols) {
+  const size_t fixed = fp_rows_smem(cols, 0, kFpWarps + 1);
+  for (int n : {kFpPerSm, kFpPerSm / 2}) {
+    const size_t room = kRowSmem / n;
+    if (fixed + 64 * sizeof(RowTilt) <= room)
+      return {n, (int)((room - fixed) / sizeof(RowTilt)) & ~1, room};
+  }
+  return {0, 0, 0};
+}
+bool fp_rows_fits(int cols) { return cols <= kZeroCols && fp_rows_resident(cols).tilts > 0; }
 
 template <int MODE, bool KAHAN>
 static cudaError_t launch_bp_rows_t(const BpArgs &a, const float *rows, int cols, cudaStream_t s) {
@@ -1077,14 +1093,21 @@ cudaError_t launch_bp_rows(int mode, const BpArgs &a, const float *rows, int col
 }
 
 cudaError_t launch_fp_rows(const FpArgs &a, float *rows, int cols, int nsm, cudaStream_t s) {
-  const int slots = fp_rows_slots(cols, a.nt);
-  const size_t smem = fp_rows_smem(cols, a.nt, slots);
+  const FpResident fit = fp_rows_resident(cols);
+  const int groups = (a.nt + fit.tilts - 1) / fit.tilts, per = (a.nt + groups - 1) / groups;
+  const int slots = fp_rows_slots(cols, per, fit.room);
+  const size_t smem = fp_rows_smem(cols, per, slots);
   cudaError_t e = cudaFuncSetAttribute(fp_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem);
   if (e != cudaSuccess) return e;
   const dim3 grid((a.v.nx + kRowFpX - 1) / kRowFpX, (a.v.nz + kRowFpZ - 1) / kRowFpZ,
                   (a.v.ny + kRowTile - 1) / kRowTile);
-  fp_rows_kernel<<<grid, kFpWarps * 32, smem, s>>>(a, rows, cols, slots, smem <= kRowSmem / kFpPerSm ? kFpPerSm * nsm : nsm);
+  for (int t = 0; t < a.nt; t += per) {
+    FpArgs g = a;
+    g.t0 = a.t0 + t;
+    g.nt = std::min(per, a.nt - t);
+    fp_rows_kernel<<<grid, kFpWarps * 32, smem, s>>>(g, rows, cols, slots, fit.per_sm * nsm);
+  }
   return cudaGetLastError();
 }
 
