@@ -278,7 +278,7 @@ BpArgs bp_args(const tr_ctx *c, float *vol, int z0, int nz, const float *img,
 // general kernels' -- and which have tiles (counted 8 sections deep) enough for
 // the SMs.  Measured (us, general / row-invariant):
 //   back-projection, pad 1.35, 128 tiles: 1024 x 1024 x 256, 61 tilts 6686 /
-//     3833; x 64, 1 tilt 320 / 147; 256 x 256 x 64, 41 tilts 91 / 68; rows 192
+//     3833; x 64, 1 tilt 168 / 147; 256 x 256 x 64, 41 tilts 91 / 68; rows 192
 //     of 256 (pad 1.33) 182 / 165, 160 of 256 (1.6) 110 / 116; 256 x 64 x 64
 //     (64 tiles, pad 2) 37 / 48;
 //   of 16-bit stacks (compensated sums; the general kernel reads the 16 bits,
@@ -289,7 +289,7 @@ BpArgs bp_args(const tr_ctx *c, float *vol, int z0, int nz, const float *img,
 //     such stack where the general kernel is the one to pad (0.85): 250 x 250 x
 //     66, 41 tilts (0.77) 161 / 103; 1000 x 1000 x 100 (0.84) 2367 / 1793;
 //   forward projection, pad 1.15, 256 tiles: 1024 x 1024 x 256, 61 tilts 8123 /
-//     5742; x 64: 41 tilts 1408 / 1280, 24 tilts 820 / 774, 8 tilts 305 / 459
+//     5742; x 64: 41 tilts 1416 / 1149, 24 tilts 829 / 741, 8 tilts 305 / 459
 //     (the tilts pass through a CTA's warps in a pipeline that must fill);
 //     256 x 256 x 64 125 / 98, x 32 (128 tiles) 99 / 112; rows 320 of 384
 //     (pad 1.2) 355 / 391.
@@ -301,12 +301,13 @@ struct RowsRule {
 };
 constexpr RowsRule kRowsBp{kTX, 1, 128, 1, 1.35}, kRowsBp16{kTX, 32, 128, 96, 1.1},
     kRowsBp16Pad{kTX, 1, 128, 1, 0.85}, kRowsFp{kFX, 24, 256, 1, 1.15};
+double tile_count(int n, int t) { return (double)((n + t - 1) / t); }
 bool rows_path(const tr_ctx *c, const RowsRule &r, int nz, int nt, cudaStream_t s) {
   if (!c->rows || nt < r.min_tilts || nz < r.min_z) return false;
-  const auto tiles = [](int n, int t) { return (double)((n + t - 1) / t); };
-  const double n = tiles(c->nx, kRowBpX) * tiles(c->ny, kRowTile) * tiles(nz, kRowBpZ);
-  const double general = tiles(c->nx, r.general_x) * r.general_x * tiles(c->ny, kTY) * kTY *
-                         tiles(nz, kTZ) * kTZ;
+  const double n =
+      tile_count(c->nx, kRowBpX) * tile_count(c->ny, kRowTile) * tile_count(nz, kRowBpZ);
+  const double general = tile_count(c->nx, r.general_x) * r.general_x * tile_count(c->ny, kTY) *
+                         kTY * tile_count(nz, kTZ) * kTZ;
   if (n < r.min_tiles || n * kRowBpX * kRowTile * kRowBpZ > r.pad * general) return false;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
@@ -315,6 +316,48 @@ bool rows_path(const tr_ctx *c, const RowsRule &r, int nz, int nt, cudaStream_t 
   }
   return cs == cudaStreamCaptureStatusNone;
 }
+// The padding says nothing of what the row kernels pay beside their walk: the
+// blend or the sums' conversion of the whole stack, whole waves of a few CTAs, and
+// for rows that are not whole 16 bytes an epilogue by single voxels.  With few
+// tilts or thin volumes that is most of a launch, so a single projection is also
+// compared by its estimated time: linear in the tilts, the waves W, the filled
+// part of them f and the stack's pixels P (millions), the general kernels' the
+// same with their waves' filled part F, and V million voxels.  Fits to 2160, 1512
+// and 2000 launches on 148 SMs (250 to 2048 columns, 128 to 1024 rows, 1 to 128
+// sections, 1 to 140 tilts), 5 to 7 % rms.  Of the launches that the bounds above
+// let pass, those slower than the general kernel by more than 3 % fall from 602 of
+// 1352 (worst 2.52 x: 250 x 384 x 64, 1 tilt, 23 / 59 us) to 31 (1.14 x), with
+// 16-bit stacks from 83 of 394 (1.77 x) to 2, projections from 99 of 1287
+// (1.26 x: 1000 x 330 x 32, 24 tilts, 156 / 196 us) to 17 (1.09 x), and the ones
+// refused that would gain 3 % are 28, 20 and 11.  SIRT's pair of projections,
+// which forms the residual between the row stacks, gains wherever the bounds let it
+// pass (516 launches from 16 sections and 24 tilts on).
+struct RowsCost {
+  double g0, gt, gft, gct, gna, gf, gv;      // general: per launch; per tilt: 1, F, whole waves,
+                                             // F without TMA; F; V
+  double r0, rt, rwt, rft, rpt, rw, rf, rna;  // rows: per launch; per tilt: 1, W, f, P; W; f;
+                                             // f of rows that are not whole 16 bytes
+  int z, per_sm, tma;                        // section tile, CTAs per SM, pixels of 16 bytes
+};
+constexpr RowsCost kCostBp{12, .30, .66, 0, .17, 2.0, .34, 15, .13, .49, .44, 2.9, 5.9, 2.7, 11,
+                           kRowBpZ, 2, 4},
+    kCostBp16{12, .31, .70, 0, .20, 2.8, .34, 18, .08, .56, .23, 3.1, 2.7, 2.2, 4.2,
+              kRowBpZ / 2, 2, 8},
+    kCostFp{18, .51, 1.4, .41, 0, 0, 0, 20, 0, .72, .81, 4.9, 8.3, 0, 0, kRowFpZ, 4, 4};
+bool rows_gain(const tr_ctx *c, const RowsRule &r, const RowsCost &k, int nz, int nt) {
+  const double F = tile_count(c->nx, r.general_x) * tile_count(c->ny, kTY) * tile_count(nz, kTZ) /
+                   (3.0 * c->nsm);
+  const double f = tile_count(c->nx, kRowBpX) * tile_count(c->ny, kRowTile) *
+                   tile_count(nz, k.z) / ((double)k.per_sm * c->nsm);
+  const double W = ceil(f), P = 1e-6 * c->nx * tile_count(c->ny, kRowTile) * kRowTile;
+  const double V = 1e-6 * c->nx * c->ny * nz;
+  const double general = k.g0 + k.gf * F + k.gv * V +
+                         nt * (k.gt + k.gft * F + k.gct * ceil(F) + (c->nx % k.tma ? k.gna * F : 0));
+  const double rows = k.r0 + nt * (k.rt + k.rwt * W + k.rft * f + k.rpt * P) + k.rw * W + k.rf * f +
+                      (c->nx % 4 ? k.rna * f : 0);
+  return rows <= 0.98 * general;
+}
+static_assert(kRowBpX == kRowFpX, "one column tile for the rules");
 static_assert(kTZ == kFTZ, "one section tile for the rule");
 // Orders `s` after the row buffers' last use, on whichever stream that was, and
 // marks their use so far on `s` as the last.
@@ -352,6 +395,7 @@ cudaError_t run_bp(tr_ctx *c, int mode, const BpArgs &a, cudaStream_t s) {
       (a.img.dtype == IMG_F32 ? rows_path(c, kRowsBp, a.v.nz, a.nt, s)
                               : rows_path(c, kRowsBp16, a.v.nz, a.nt, s) ||
                                     rows_path(c, kRowsBp16Pad, a.v.nz, a.nt, s)) &&
+      rows_gain(c, kRowsBp, a.img.dtype == IMG_F32 ? kCostBp : kCostBp16, a.v.nz, a.nt) &&
       bp_rows_fits(c->rbp_cols, a.nt) &&
       scratch_try(c, (void **)&c->rows_d,
                   row_stack_floats(c->nx, c->ny, a.nt, c->rbp_cols) * sizeof(float))) {
@@ -407,7 +451,8 @@ FpArgs fp_args(const tr_ctx *c, const float *vol, int z0, int nz, float *val,
 tr_status run_fp(tr_ctx *c, const FpArgs &a, cudaStream_t s) {
   if (!c->deterministic) {
     const size_t rb = row_stack_floats(c->nx, c->ny, a.nt, c->rfp_cols) * sizeof(float);
-    if (rows_path(c, kRowsFp, a.v.nz, a.nt, s) && fp_rows_fits(c->rfp_cols) &&
+    if (rows_path(c, kRowsFp, a.v.nz, a.nt, s) && rows_gain(c, kRowsFp, kCostFp, a.v.nz, a.nt) &&
+        fp_rows_fits(c->rfp_cols) &&
         scratch_try(c, (void **)&c->rowsum_d, rb)) {
       const FpArgs f = own_tilts(a);
       TR_CUDA(c, rows_acquire(c, s));
