@@ -327,9 +327,9 @@ bool rows_path(const tr_ctx *c, const RowsRule &r, int nz, int nt, cudaStream_t 
 // sections, 1 to 140 tilts), 5 to 7 % rms.  Of the launches that the bounds above
 // let pass, those slower than the general kernel by more than 3 % fall from 602 of
 // 1352 (worst 2.52 x: 250 x 384 x 64, 1 tilt, 23 / 59 us) to 31 (1.14 x), with
-// 16-bit stacks from 83 of 394 (1.77 x) to 2, projections from 99 of 1287
+// 16-bit stacks from 83 of 394 (1.77 x) to 3 (1.10 x), projections from 99 of 1287
 // (1.26 x: 1000 x 330 x 32, 24 tilts, 156 / 196 us) to 17 (1.09 x), and the ones
-// refused that would gain 3 % are 28, 20 and 11.  SIRT's pair of projections,
+// refused that would gain 3 % are 25, 18 and 9.  SIRT's pair of projections,
 // which forms the residual between the row stacks, gains wherever the bounds let it
 // pass (516 launches from 16 sections and 24 tilts on).
 struct RowsCost {
@@ -355,7 +355,7 @@ bool rows_gain(const tr_ctx *c, const RowsRule &r, const RowsCost &k, int nz, in
                          nt * (k.gt + k.gft * F + k.gct * ceil(F) + (c->nx % k.tma ? k.gna * F : 0));
   const double rows = k.r0 + nt * (k.rt + k.rwt * W + k.rft * f + k.rpt * P) + k.rw * W + k.rf * f +
                       (c->nx % 4 ? k.rna * f : 0);
-  return rows <= 0.98 * general;
+  return rows <= (f > 4 ? 1.0 : 0.98) * general;  // the fits are closer for many waves
 }
 static_assert(kRowBpX == kRowFpX, "one column tile for the rules");
 static_assert(kTZ == kFTZ, "one section tile for the rule");
