@@ -3,7 +3,6 @@
 #pragma once
 
 #include <cuda.h>
-#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -90,8 +89,5 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
       "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(m))
       : "memory");
 }
-
-// cuTensorMapEncodeTiled, or nullptr where the driver has none (tr_kernels.cu).
-PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder();
 
 }  // namespace trb

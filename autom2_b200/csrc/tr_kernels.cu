@@ -32,6 +32,7 @@
 // the two rows are blended while staging and the inner loop is one table
 // read and one FMA per voxel and tilt.
 #include <cuda.h>
+#include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <stdint.h>
@@ -1610,7 +1611,7 @@ static cudaError_t launch_bp_t(const BpArgs &a, cudaStream_t s) {
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link
 // against the driver library).
-PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
+static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
   static bool tried = false;
   if (!tried) {
