@@ -1237,13 +1237,13 @@ tr_status tr_sart(tr_ctx *c, const float *proj, float *vol, int iters, float gam
                           "reprojection")))
     return st;
   if ((st = ensure_wt(c, s))) return st;
-  const int steps = iters * c->nt;
+  const long long steps = (long long)iters * c->nt;
   // Sweeps: the deterministic flush has no such form, a single tilt's residual
   // plane is in use, and two of a wide window's tables would not fit.
   const bool sweep = !c->deterministic && c->nt > 1 &&
                      sart_tables(c->sep, c->fw, c->fh) <= kSmemMax / 2;
-  for (int i = 0; i < steps; ++i) {
-    const int t = i % c->nt;
+  for (long long i = 0; i < steps; ++i) {
+    const int t = (int)(i % c->nt);
     float *vt = c->val_d + plane * t;
     // The volume's projection at the first tilt; later ones come with the update
     // of the tilt before.
@@ -1254,7 +1254,7 @@ tr_status tr_sart(tr_ctx *c, const float *proj, float *vol, int iters, float gam
     }
     TR_CUDA(c, launch_resid(proj + plane * t, vt, c->wt_d + plane * t, plane, c->nsm, s));
     if (i + 1 < steps && sweep) {
-      const int n = (i + 1) % c->nt;
+      const int n = (int)((i + 1) % c->nt);
       // the next iteration's, of which the last tilt's is this step's residual
       if (n == 0)
         TR_CUDA(c, cudaMemsetAsync(c->val_d, 0, (c->nt - 1) * plane * sizeof(float), s));
