@@ -277,22 +277,22 @@ BpArgs bp_args(const tr_ctx *c, float *vol, int z0, int nz, const float *img,
 // does not outweigh its gain -- `pad` bounds the padded voxels relative to the
 // general kernels' -- and which have tiles (counted 8 sections deep) enough for
 // the SMs.  Measured (us, general / row-invariant):
-//   back-projection, pad 1.35, 128 tiles: 1024 x 1024 x 256, 61 tilts 6686 /
-//     3833; x 64, 1 tilt 168 / 147; 256 x 256 x 64, 41 tilts 91 / 68; rows 192
-//     of 256 (pad 1.33) 182 / 165, 160 of 256 (1.6) 110 / 116; 256 x 64 x 64
-//     (64 tiles, pad 2) 37 / 48;
+//   back-projection, pad 1.35, 128 tiles: 1024 x 1024 x 256, 61 tilts 6498 /
+//     3852; x 64, 1 tilt 165 / 156; 256 x 256 x 64, 41 tilts 95 / 77; rows 192
+//     of 256 (pad 1.33) 83 / 74, 160 of 256 (1.6) 75 / 73; 256 x 64 x 64 (64
+//     tiles, pad 2) 42 / 55;
 //   of 16-bit stacks (compensated sums; the general kernel reads the 16 bits,
 //     the row stack is FP32 and its blend must be shared by sections enough),
-//     pad 1.1, 32 tilts, 96 sections: 1024 x 1024 x 256, 61 tilts 6905 / 6172,
-//     x 64, 24 tilts 762 / 780; 256 x 256 x 64, 41 tilts 91 / 97; 512 x 200 x 64
-//     (pad 1.28) 130 / 166; 1024 x 1024 x 64, 8 tilts (pad 1) 330 / 356.  Any
+//     pad 1.1, 32 tilts, 96 sections: 1024 x 1024 x 256, 61 tilts 6916 / 6184,
+//     x 64, 24 tilts 773 / 786; 256 x 256 x 64, 41 tilts 99 / 106; 512 x 200 x 64
+//     (pad 1.28) 140 / 176; 1024 x 1024 x 64, 8 tilts (pad 1) 340 / 365.  Any
 //     such stack where the general kernel is the one to pad (0.85): 250 x 250 x
-//     66, 41 tilts (0.77) 161 / 103; 1000 x 1000 x 100 (0.84) 2367 / 1793;
-//   forward projection, pad 1.15, 256 tiles: 1024 x 1024 x 256, 61 tilts 8123 /
-//     5742; x 64: 41 tilts 1416 / 1149, 24 tilts 829 / 741, 8 tilts 305 / 459
+//     66, 41 tilts (0.77) 171 / 111; 1000 x 1000 x 100, 61 tilts (0.84) 3398 / 2549;
+//   forward projection, pad 1.15, 256 tiles: 1024 x 1024 x 256, 61 tilts 8132 /
+//     5551; x 64: 41 tilts 1417 / 1191, 24 tilts 828 / 755, 8 tilts 313 / 361
 //     (the tilts pass through a CTA's warps in a pipeline that must fill);
-//     256 x 256 x 64 125 / 98, x 32 (128 tiles) 99 / 112; rows 320 of 384
-//     (pad 1.2) 355 / 391.
+//     256 x 256 x 64, 41 tilts 134 / 108, x 32 (128 tiles) 77 / 84; 1024 x 320 x
+//     64, 24 tilts (pad 1.2) 286 / 318.
 // Not under stream capture, whose graphs must not hold a buffer that the
 // context may drop.
 struct RowsRule {
@@ -322,8 +322,9 @@ bool rows_path(const tr_ctx *c, const RowsRule &r, int nz, int nt, cudaStream_t 
 // tilts or thin volumes that is most of a launch, so a single projection is also
 // compared by its estimated time: linear in the tilts, the waves W, the filled
 // part of them f and the stack's pixels P (millions), the general kernels' the
-// same with their waves' filled part F, and V million voxels.  Fits to 2160, 1512
-// and 2000 launches on 148 SMs (250 to 2048 columns, 128 to 1024 rows, 1 to 128
+// same with their waves' filled part F, and V million voxels, which at HBM's pace
+// (a little less per tilt) bounds large ones of few tilts.  Fits to 2160, 1512 and
+// 2000 launches on 148 SMs (250 to 2048 columns, 128 to 1024 rows, 1 to 128
 // sections, 1 to 140 tilts), 5 to 7 % rms.  Of the launches that the bounds above
 // let pass, those slower than the general kernel by more than 3 % fall from 602 of
 // 1352 (worst 2.52 x: 250 x 384 x 64, 1 tilt, 23 / 59 us) to 31 (1.14 x), with
@@ -333,17 +334,17 @@ bool rows_path(const tr_ctx *c, const RowsRule &r, int nz, int nt, cudaStream_t 
 // which forms the residual between the row stacks, gains wherever the bounds let it
 // pass (516 launches from 16 sections and 24 tilts on).
 struct RowsCost {
-  double g0, gt, gft, gct, gna, gf, gv;      // general: per launch; per tilt: 1, F, whole waves,
-                                             // F without TMA; F; V
+  double g0, gt, gft, gct, gna, gf, gv, gm;  // general: per launch; per tilt: 1, F, whole waves,
+                                             // F without TMA; F; V; V at least (HBM)
   double r0, rt, rwt, rft, rpt, rw, rf, rna;  // rows: per launch; per tilt: 1, W, f, P; W; f;
                                              // f of rows that are not whole 16 bytes
   int z, per_sm, tma;                        // section tile, CTAs per SM, pixels of 16 bytes
 };
-constexpr RowsCost kCostBp{12, .30, .66, 0, .17, 2.0, .34, 15, .13, .49, .44, 2.9, 5.9, 2.7, 11,
+constexpr RowsCost kCostBp{12, .30, .66, 0, .17, 2.0, .34, 2.2, 15, .13, .49, .44, 2.9, 5.9, 2.7, 11,
                            kRowBpZ, 2, 4},
-    kCostBp16{12, .31, .70, 0, .20, 2.8, .34, 18, .08, .56, .23, 3.1, 2.7, 2.2, 4.2,
+    kCostBp16{12, .31, .70, 0, .20, 2.8, .34, 2.6, 18, .08, .56, .23, 3.1, 2.7, 2.2, 4.2,
               kRowBpZ / 2, 2, 8},
-    kCostFp{18, .51, 1.4, .41, 0, 0, 0, 20, 0, .72, .81, 4.9, 8.3, 0, 0, kRowFpZ, 4, 4};
+    kCostFp{18, .51, 1.4, .41, 0, 0, 0, 0, 20, 0, .72, .81, 4.9, 8.3, 0, 0, kRowFpZ, 4, 4};
 bool rows_gain(const tr_ctx *c, const RowsRule &r, const RowsCost &k, int nz, int nt) {
   const double F = tile_count(c->nx, r.general_x) * tile_count(c->ny, kTY) * tile_count(nz, kTZ) /
                    (3.0 * c->nsm);
@@ -351,8 +352,10 @@ bool rows_gain(const tr_ctx *c, const RowsRule &r, const RowsCost &k, int nz, in
                    tile_count(nz, k.z) / ((double)k.per_sm * c->nsm);
   const double W = ceil(f), P = 1e-6 * c->nx * tile_count(c->ny, kRowTile) * kRowTile;
   const double V = 1e-6 * c->nx * c->ny * nz;
-  const double general = k.g0 + k.gf * F + k.gv * V +
-                         nt * (k.gt + k.gft * F + k.gct * ceil(F) + (c->nx % k.tma ? k.gna * F : 0));
+  const double general =
+      std::max(k.gm * V * (1 + .07 * nt),
+               k.g0 + k.gf * F + k.gv * V +
+                   nt * (k.gt + k.gft * F + k.gct * ceil(F) + (c->nx % k.tma ? k.gna * F : 0)));
   const double rows = k.r0 + nt * (k.rt + k.rwt * W + k.rft * f + k.rpt * P) + k.rw * W + k.rf * f +
                       (c->nx % 4 ? k.rna * f : 0);
   return rows <= (f > 4 ? 1.0 : 0.98) * general;  // the fits are closer for many waves

@@ -132,3 +132,21 @@ def test_compensated_sums_at_the_groups_of_tilts(fresh, restatement, nt):
     fresh.backproject_lp(q, scale, v)
     assert fresh.scratch_bytes > held
     assert O.rel_l2(v.cpu().numpy(), R.backproject(g, c8, exact, vol, fp64=True)) < 6e-7
+
+
+@pytest.mark.parametrize("resid", ["f32", "f16"])
+@pytest.mark.parametrize("layout,depth", [(0, 32), (1, 64), (0, 96)])
+def test_slabs_of_sections(fresh, restatement, layout, depth, resid):
+    """z-slab SIRT where single projections and whole volumes take the row-invariant
+    kernels.  FP32 residuals to the parity bar; FP16 ones keep 11 bits of each pixel's
+    residual, of which a voxel averages 41: to 1e-4."""
+    R = restatement
+    nx, ny, nt, th = 250, 256, 41, 96
+    c8, proj, vol, org, g = _case(R, nx, ny, nt, th, layout)
+    want = R.sirt(g, c8, proj, vol, 2, 0.5, fp64=True)
+    fresh.set_problem(nx, ny, nt, th, c8, layout, org)
+    p = torch.from_numpy(proj).cuda()
+    for v in (torch.from_numpy(vol.copy()).cuda(), torch.from_numpy(vol.copy()).pin_memory()):
+        fresh.sirt_zslabs(p, v, 2, 0.5, depth, resid_dtype=resid)
+        torch.cuda.synchronize()
+        assert O.rel_l2(v.cpu().numpy(), want) < (TOL if resid == "f32" else 1e-4)
