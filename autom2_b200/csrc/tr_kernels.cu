@@ -1150,8 +1150,8 @@ __device__ __forceinline__ float resid_of(float p, float val, float w) {
   if (w != 0.f) val /= w;
   return p - val;
 }
-// Bound by HBM: four pixels per access where the pointers allow (61 x 1024 x
-// 1024 pixels; 41 x 512 x 512 45 -> 28 us).
+// Bound by HBM: four pixels per access where the pointers allow (41 x 512 x 512
+// pixels 45 -> 28 us).
 __global__ void __launch_bounds__(256)
     resid_kernel(const float *__restrict__ p, float *val, const float *__restrict__ wt, size_t n) {
   const size_t first = blockIdx.x * (size_t)blockDim.x + threadIdx.x,

@@ -247,8 +247,9 @@ constexpr int kLag = 4;  // a stage is refilled kLag tilts after its use
 // registers a thread, which spills.)
 //
 // Bound by issue and by latency at 16 warps per SM (128 registers: 64 sums):
-// 61 % of issue slots, 5.5 instructions per voxel and tilt where the general
-// kernel takes 7 with one row per table entry; shared memory 42 %, L2 17 %.
+// 63 % of issue slots, 5.2 instructions per voxel and tilt where the general
+// kernel takes 7 with one row per table entry, 75 % of the shared-memory
+// wavefronts.
 // 1024 x 1024 x 256 voxels, 61 tilts: 3.83 ms with the row stack's 0.15 ms,
 // from 6.69 ms by the general kernel (4.3e12 from 2.4e12 voxel-tilts/s).
 //

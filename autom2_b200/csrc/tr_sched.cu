@@ -3,10 +3,9 @@
 // The reference reconstructs one tilt series per process run (TiltRec-cuda /
 // TiltRec-mpi launched by the GUI's command chain); it has no batching or
 // serving.  This scheduler keeps many jobs device-resident and advances all of
-// them together: every step is one table of work items run by four launches
-// (zero, persistent forward projection, residual, FP16 residual maxima and
-// conversion, persistent back-projection)
-// captured once in a CUDA graph and replayed with a new table each step.  A
+// them together: every step is one table of work items run by five launches
+// (zero, persistent forward projection, residual with the FP16 ones' maxima, FP16
+// conversion, persistent back-projection) captured once in a CUDA graph and replayed with a new table each step.  A
 // job's SIRT iterations are consecutive steps; a WBP job (or the WBP start of
 // a WBP-then-SIRT job) is one back-projection item.
 //
@@ -77,7 +76,7 @@ struct Job {
   const float *ps = nullptr, *rs = nullptr;
   BatchBp bp_norm{}, bp_sirt{};
   BatchFp fp{};
-  BpArgs a_norm{}, a_sirt{};  // the same work for the per-job kernels
+  BpArgs a_norm{}, a_sirt{};  // the same work for launches of one job
   double work = 0;            // remaining voxel-projection updates
   size_t smem_norm = 0, smem_sirt = 0;
   // progress
@@ -457,7 +456,7 @@ void release(tr_sched *S, Job &j, cudaStream_t s) {
   S->pool_since = now_s();
 }
 
-// Captures the four launches of a step over table b.
+// Captures the five launches of a step over table b.
 tr_status capture(tr_sched *S, int b) {
   cudaGraph_t g = nullptr;
   SCHED_CUDA(S, cudaStreamBeginCapture(S->s, cudaStreamCaptureModeThreadLocal));
@@ -503,8 +502,8 @@ double srpt_key(const tr_sched *S, const Job &j, double now) {
 }
 
 // TR_SCHED_SRPT step: the next unit of the ready job with the least remaining
-// work (its WBP back-projection, or one SIRT iteration) through the per-job
-// kernels the context path runs.  At most two steps are in flight, so a job
+// work (its WBP back-projection, or one SIRT iteration) through the general
+// kernels, one job a launch.  At most two steps are in flight, so a job
 // that becomes ready is considered within one step.
 tr_status launch_job_step(tr_sched *S, bool *launched) {
   Job *j = nullptr;

@@ -97,8 +97,14 @@ tr_status tr_geometry_from_angles(const float *angles_deg, int ntilt,
  * allocates only when a larger one arrives; a buffer that three problems in
  * a row have not used is freed at the next tr_set_problem, and under a
  * budget, or when the device is short of memory, buffers the current problem
- * has not used are released first.  tr_scratch_bytes reports the budgeted buffers held;
- * tr_destroy frees everything. */
+ * has not used are released first.  Projections of geometries without XTILT
+ * and in-plane rotation also take row stacks from it -- one or two more of the
+ * size of the projection stack, by any call that projects, tr_backproject and
+ * tr_forward_project included -- where the budget and the device have the room;
+ * they are dropped for any buffer that a call cannot do without, and without
+ * them (a budget bounds them) the calls run other, slower kernels.
+ * tr_scratch_bytes reports the budgeted buffers held; tr_destroy frees
+ * everything. */
 tr_status tr_create(int device, size_t hbm_budget, tr_ctx **out);
 tr_status tr_destroy(tr_ctx *ctx);
 const char *tr_last_error(const tr_ctx *ctx);
@@ -240,7 +246,9 @@ tr_status tr_quantize(tr_ctx *ctx, const float *proj_dev, int dtype,
                       void *out_dev, float *scale_dev, void *stream);
 
 /* Back-projection (as tr_backproject) from a 16-bit stack; the FP32 sums
- * over tilts are compensated (Kahan) per voxel. */
+ * over tilts are compensated (Kahan) per voxel, by groups: up to 16 or 32 tilts
+ * (by the kernel) are summed plainly, and each group's sum joins the voxel's
+ * total by one compensated addition. */
 tr_status tr_backproject_lp(tr_ctx *ctx, const void *proj_dev, int dtype,
                             const float *scale_dev, float *vol_dev, int z0,
                             int nz, void *stream);
@@ -251,8 +259,8 @@ tr_status tr_backproject_lp(tr_ctx *ctx, const void *proj_dev, int dtype,
  * power-of-two scales, recomputed every iteration (the residual's range is
  * not the stack's: after a WBP start it can be far larger); or BF16 (float's
  * range, no scale).  The reprojection, weights and volume stay FP32; the
- * residual back-projection sums are compensated per voxel when the residual
- * is 16-bit. */
+ * residual back-projection sums are compensated per voxel, as those of
+ * tr_backproject_lp, when the residual is 16-bit. */
 tr_status tr_sirt_lp(tr_ctx *ctx, const void *proj_dev, int proj_dtype,
                      const float *scale_dev, int resid_dtype, float *vol_dev,
                      int iters, float gamma, void *stream);
@@ -269,8 +277,9 @@ tr_status tr_sirt_lp(tr_ctx *ctx, const void *proj_dev, int proj_dtype,
  * the call then returns when the volume is written back.  Otherwise `vol` is
  * the device volume and the call is ordered on `stream`.  depth: sections per
  * slab, rounded down to a multiple of 32 (at least 32; the whole thickness
- * when larger).  Results equal tr_sirt / tr_sirt_lp up to the order of the
- * forward projection's float atomic adds.  Device memory: two reprojections
+ * when larger).  Results equal tr_sirt / tr_sirt_lp up to rounding: the order
+ * of the forward projection's float additions, and the kernels that a slab's
+ * depth suits.  Device memory: two reprojections
  * (ntilt*ny*nx floats each), the weights, and with a host volume three slabs
  * of depth*ny*nx floats. */
 tr_status tr_sirt_zslabs(tr_ctx *ctx, const void *proj_dev, int proj_dtype,
@@ -335,8 +344,10 @@ tr_status tr_autotune_zslab(tr_ctx *ctx, const void *proj_dev, int proj_dtype,
  *  - TR_SCHED_SRPT: shortest remaining work first.  Admission takes the
  *    queued job with the least work that fits; each step runs the next unit
  *    (WBP back-projection or SIRT iteration) of the ready job with the least
- *    work left, through the same per-job kernels as tr_sirt / tr_wbp
- *    (optionally aged: tr_sched_set_aging).
+ *    work left, by itself, through the general kernels of tr_sirt / tr_wbp
+ *    (optionally aged: tr_sched_set_aging).  A context may run a large series
+ *    of a geometry without XTILT and rotation faster: its row-invariant
+ *    kernels are not part of the scheduler's steps.
  * A background thread drives the steps; calls are thread-safe.
  * Results do not depend on the other jobs in the mix beyond the order of the
  * forward projection's float atomic adds (as for a job run alone).  Images
