@@ -5,9 +5,10 @@
 // serving.  This scheduler keeps many jobs device-resident and advances all of
 // them together: every step is one table of work items run by five launches
 // (zero, persistent forward projection, residual with the FP16 ones' maxima, FP16
-// conversion, persistent back-projection) captured once in a CUDA graph and replayed with a new table each step.  A
-// job's SIRT iterations are consecutive steps; a WBP job (or the WBP start of
-// a WBP-then-SIRT job) is one back-projection item.
+// conversion, persistent back-projection) captured once in a CUDA graph and
+// replayed with a new table each step.  A job's SIRT iterations are consecutive
+// steps; a WBP job (or the WBP start of a WBP-then-SIRT job) is one
+// back-projection item.
 //
 // Jobs are admitted in submission order while their device memory fits the
 // HBM budget.  Admission (upload, 16-bit quantisation of the projections,
